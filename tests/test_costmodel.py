@@ -107,6 +107,30 @@ def test_gpu_adam_and_predict_match_oracle(engine, cuda):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("n", [3, 4, 64, 607, 609, 1216, 1217, 4864, 4881, 14593])
+def test_gpu_tiles_of_every_shape_match_oracle(engine, cuda, n):
+    """Minibatches at the edges of the tile kernels (one, two and four samples per
+    thread, several tiles per CTA, the thread-per-row prediction): fp32 chains of at
+    most 64 products per layer and sums over n samples, against fp64."""
+    import torch
+    from ttv_gb300 import batch as B
+    rng = np.random.default_rng(n)
+    p = rand_params(n)
+    x = rng.standard_normal((n, M.IN)).astype(np.float32)
+    y = rng.standard_normal(n).astype(np.float32)
+    dp, dx, dy = (torch.from_numpy(t).cuda() for t in (p, x, y))
+    loss, grad = B.mlp_loss_grad(dp, dx, dy)
+    L, g = M.loss_grad(p, x, y)
+    assert abs(float(loss) - L) <= 1e-4 * max(1, abs(L))
+    gg = grad.cpu().numpy().astype(np.float64)
+    assert np.max(np.abs(gg - g)) <= 2e-4 * (np.max(np.abs(g)) + 1e-12)
+    again = B.mlp_loss_grad(dp, dx, dy)
+    assert torch.equal(again[0], loss) and torch.equal(again[1], grad)
+    ref, _ = M.forward(p, x)
+    np.testing.assert_allclose(B.mlp_predict(dp, dx).cpu().numpy(), ref, rtol=1e-4, atol=1e-4)
+
+
+@pytest.mark.gpu
 def test_gpu_training_fits_a_known_function(engine, cuda):
     """Training with the engine's kernels drives the loss down on y = f(x)."""
     import torch

@@ -208,7 +208,7 @@ __global__ void __launch_bounds__(256) batch_select(BProb* __restrict__ pr, int 
         for (int i = 0; i < NFEAT; ++i) x[i] = pr[pi].feat[i];
 #pragma unroll
         for (int i = 0; i < NVARIANT; ++i) x[NFEAT + i] = (i == v) ? 1.f : 0.f;
-        score = mlp_forward<false>(sw, x, nullptr, nullptr, nullptr);
+        score = mlp_forward(sw, x);
     }
     int best = v;
     const int h = pi < n ? pr[pi].heuristic : 0;

@@ -25,11 +25,8 @@ constexpr int OFF_W4 = OFF_B3 + MLP_H;
 constexpr int OFF_B4 = OFF_W4 + MLP_H;
 constexpr int MLP_PARAMS = OFF_B4 + 1;
 
-// Forward pass of one input row; keeps the activations when `keep` is set
-// (training).  `w` may point to global or shared memory.
-template <bool KEEP>
-__device__ __forceinline__ float mlp_forward(const float* __restrict__ w, const float* x, float* a1,
-                                             float* a2, float* a3)
+// Forward pass of one input row; `w` may point to global or shared memory.
+__device__ __forceinline__ float mlp_forward(const float* __restrict__ w, const float* x)
 {
     float h1[MLP_H], h2[MLP_H];
 #pragma unroll 4
@@ -38,7 +35,6 @@ __device__ __forceinline__ float mlp_forward(const float* __restrict__ w, const 
 #pragma unroll
         for (int i = 0; i < MLP_IN; ++i) z = fmaf(x[i], w[OFF_W1 + i * MLP_H + j], z);
         h1[j] = z > 0.f ? z : 0.f;
-        if (KEEP) a1[j] = z;
     }
 #pragma unroll 4
     for (int j = 0; j < MLP_H; ++j) {
@@ -46,7 +42,6 @@ __device__ __forceinline__ float mlp_forward(const float* __restrict__ w, const 
 #pragma unroll
         for (int i = 0; i < MLP_H; ++i) z = fmaf(h1[i], w[OFF_W2 + i * MLP_H + j], z);
         h2[j] = z > 0.f ? z : 0.f;
-        if (KEEP) a2[j] = z;
     }
     float out = w[OFF_B4];
 #pragma unroll 4
@@ -54,7 +49,6 @@ __device__ __forceinline__ float mlp_forward(const float* __restrict__ w, const 
         float z = w[OFF_B3 + j];
 #pragma unroll
         for (int i = 0; i < MLP_H; ++i) z = fmaf(h2[i], w[OFF_W3 + i * MLP_H + j], z);
-        if (KEEP) a3[j] = z;
         out = fmaf(z > 0.f ? z : 0.f, w[OFF_W4 + j], out);
     }
     return out;
