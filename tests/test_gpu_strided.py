@@ -157,3 +157,95 @@ def test_vector_forms(engine, cuda):
                 absn = torch.tensordot(A.double().abs(), b.double().abs(), dims=([q - 1], [0]))
                 bar = 1e-5 if dt == torch.float32 else 1e-13
                 assert ((c.double() - ref).abs() / absn.clamp_min(1e-300)).max().item() <= bar, (dt, shape, q)
+
+
+# memory order of the base (slowest first); the last extent is padded
+SPLIT_SHAPES = [(2, 3, 2), (3, 5000, 7), (1, 90000, 4), (30000, 6), (5, 70001), (700, 33, 64), (1300, 1381),
+                (4, 3, 100000), (17, 2, 4096), (4099, 3, 5, 8), (2, 400, 640), (61, 16, 500)]
+
+
+@pytest.mark.parametrize("pad", [1, 4])
+@pytest.mark.parametrize("dt", [np.float32, np.float64], ids=["fp32", "fp64"])
+@pytest.mark.parametrize("shape", SPLIT_SHAPES, ids=["x".join(map(str, s)) for s in SPLIT_SHAPES])
+def test_shared_contractions(engine, orc, cuda, shape, dt, pad):
+    """Every way the contracted mode is shared (warps, clusters, segments of the grid), loads of
+    one element and of 16 bytes, several rows or columns per thread: every mode of padded views,
+    into contiguous and into padded, permuted outputs.  Truth in double-double.  Bars: Kahan's
+    two roundings per product and the result's (fp32: 4 x 2^-24); one rounding per product and
+    the result's (fp64: 4 x 2^-53), both of sum |a b|."""
+    import torch
+    tdt = torch.float32 if dt == np.float32 else torch.float64
+    g = torch.Generator(device=cuda)
+    g.manual_seed(len(shape) * 1000 + shape[-1] + pad)
+    base = torch.rand(*shape[:-1], shape[-1] + pad, generator=g, device=cuda, dtype=tdt) * 2 - 1
+    A = base[..., :shape[-1]]
+    p = len(shape)
+    bar = 4 * 2.0 ** -24 if dt == np.float32 else 4 * 2.0 ** -53
+    dense = A.contiguous().cpu().numpy().ravel()
+    for q in range(1, p + 1):
+        b = torch.rand(shape[q - 1], generator=g, device=cuda, dtype=tdt) * 2 - 1
+        S, nq, P = int(np.prod(shape[:q - 1])), shape[q - 1], int(np.prod(shape[q:]))
+        ref, absn = orc.truth(S, nq, P, dense, b.cpu().numpy())
+        oshape = [n for m, n in enumerate(shape) if m != q - 1]
+        wide = torch.full([n + 1 for n in reversed(oshape)], 7.0, device=cuda, dtype=tdt)
+        out = wide.permute(*range(p - 2, -1, -1))[tuple(slice(0, n) for n in oshape)]
+        for c in (engine.ttv_view(q, A, b), engine.ttv_view(q, A, b, out=out)):
+            got = c.contiguous().cpu().numpy().ravel()
+            assert orc.rel_error(got, ref, absn) <= bar, (shape, q, dt, pad)
+        rest = wide.clone()
+        rest.permute(*range(p - 2, -1, -1))[tuple(slice(0, n) for n in oshape)].fill_(7.0)
+        assert (rest == 7.0).all()
+
+
+@pytest.mark.parametrize("kind", ["growing", "falling", "zeros", "huge", "tiny", "mixed", "cancelling"])
+@pytest.mark.parametrize("row", [True, False], ids=["row", "col"])
+def test_fp64_exponent_windows(engine, orc, cuda, kind, row):
+    """The fixed-point sums' window: products that outgrow it, fall below it, vanish, sit at the
+    ends of the exponent range or cancel; bar: one rounding per product and the result's, of
+    sum |a b| (and of the smallest normal number)."""
+    import torch
+    n, m = 3000, 41
+    rng = np.random.default_rng(11)
+    a = rng.uniform(-1, 1, (m, n))
+    if kind == "growing":
+        a *= np.exp2(np.linspace(-300, 300, n))
+    elif kind == "falling":
+        a *= np.exp2(np.linspace(300, -300, n))
+    elif kind == "zeros":
+        a[rng.uniform(size=a.shape) < 0.9] = 0.0
+        a[5] = 0.0
+    elif kind == "huge":
+        a *= 2.0 ** 1009
+    elif kind == "tiny":
+        a *= 2.0 ** -1020
+    elif kind == "mixed":
+        a *= np.exp2(rng.uniform(-200, 200, a.shape))
+    else:
+        a[:, 1::2] = -a[:, 0::2]
+    b = np.ones(n) if kind == "cancelling" else rng.uniform(-1, 1, n)
+    buf = np.zeros((m, n + 3))
+    buf[:, :n] = a
+    A = torch.from_numpy(buf).to(cuda)[:, :n]
+    if not row:
+        A = torch.from_numpy(np.ascontiguousarray(buf.T)).to(cuda)[:n].T   # contracted mode strided
+        A = torch.nn.functional.pad(A.T, (0, 3))[:, :m].T
+    c = engine.ttv_view(2, A, torch.from_numpy(b).to(cuda)).cpu().numpy()
+    import fractions
+    for i in range(0, m, 5):
+        terms = [fractions.Fraction(x) * fractions.Fraction(y) for x, y in zip(a[i], b)]
+        exact, absn = sum(terms), sum(abs(t) for t in terms)
+        bar = absn * fractions.Fraction(4, 2 ** 53) + n * fractions.Fraction(1, 2 ** 1074)
+        assert abs(fractions.Fraction(float(c[i])) - exact) <= bar, (kind, i)
+
+
+def test_fp64_nonfinite_products(engine, cuda):
+    """Infinities and NaNs among the products reach their output and no other."""
+    import torch
+    a = torch.rand(37, 500, device=cuda, dtype=torch.float64)
+    b = torch.rand(500, device=cuda, dtype=torch.float64)
+    a[3, 77], a[8, 2], a[20, 499] = float("inf"), float("nan"), float("-inf")
+    for A in (torch.nn.functional.pad(a, (0, 3))[:, :500], torch.nn.functional.pad(a.T, (0, 3))[:, :37].T):
+        c = engine.ttv_view(2, A, b)
+        bad = torch.zeros(37, dtype=torch.bool, device=cuda)
+        bad[[3, 8, 20]] = True
+        assert not torch.isfinite(c[bad]).any() and torch.isfinite(c[~bad]).all()

@@ -1120,62 +1120,31 @@ int tlibg_ttv_strided(int dtype, size_t q, size_t p, const void* a, const size_t
     if (!dev_info().ok) return fail(TLIBG_ERR_CUDA, "tlibg: no usable CUDA device");
     if (int st = check_device_pointers(a, b, c)) return st;
 
-    // modes other than q, A-stride order; C's mode r (0-based) is A's mode r or r + 1
-    GSArgs k{};
+    // modes other than q; C's mode r (0-based) is A's mode r or r + 1
+    GSPlan pl;
     std::vector<std::tuple<size_t, size_t, size_t>> modes;   // (wa, extent, wc)
     for (size_t m = 0; m < p; ++m) {
         if (m == q - 1) continue;
         const size_t cm = m < q - 1 ? m : m - 1;
         if (na[m] > 1) modes.emplace_back(wa[m], na[m], wc[cm]);
     }
-    std::sort(modes.begin(), modes.end());
-    k.nm = (int)modes.size();
-    k.outputs = 1;
-    for (int r = 0; r < k.nm; ++r) {
-        k.wa[r] = std::get<0>(modes[r]);
-        k.ext[r] = std::get<1>(modes[r]);
-        k.wc[r] = std::get<2>(modes[r]);
-        k.outputs *= k.ext[r];
-    }
-    k.a = a;
-    k.b = b;
-    k.c = c;
-    k.nq = na[q - 1];
-    k.waq = na[q - 1] > 1 ? wa[q - 1] : 0;
-    k.wb = wb;
-    const bool row = k.nm == 0 || (k.nq > 1 && k.waq <= k.wa[0]);
-    k.group = (uint32_t)std::max(1, std::min(32, pow2_floor(std::max<uint64_t>(1, k.nq / 16))));
+    gs_modes(std::move(modes), &pl.k);
+    pl.k.a = a;
+    pl.k.b = b;
+    pl.k.c = c;
+    pl.k.nq = na[q - 1];
+    pl.k.waq = na[q - 1] > 1 ? wa[q - 1] : 0;
+    pl.k.wb = wb;
     const int sms = dev_info().sms;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    // 16-byte forms where the view allows them
-    const uint64_t V = 16 / (dtype == F64 ? 8 : 4);
-    bool others_on_grid = (reinterpret_cast<uintptr_t>(a) % 16) == 0;
-    for (int r = 0; r < k.nm; ++r) others_on_grid = others_on_grid && k.wa[r] % V == 0;
-    const bool row_vec = row && k.waq == 1 && k.nq % V == 0 && wb == 1 &&
-                         (reinterpret_cast<uintptr_t>(b) % 16) == 0 && others_on_grid;
-    bool col_vec = !row && k.nm > 0 && k.wa[0] == 1 && k.ext[0] % V == 0 &&
-                   (reinterpret_cast<uintptr_t>(a) % 16) == 0 && k.waq % V == 0;
-    for (int r = 1; r < k.nm; ++r) col_vec = col_vec && k.wa[r] % V == 0;
-    // one thread per V outputs only while the outputs alone still fill the GPU (the
-    // column forms take no split of n_q): measured on 2^26-element padded views,
-    // 131072 outputs over 512 rows ran 1.8 TB/s with V per thread, 4.1 with one
-    col_vec = col_vec && k.outputs / V >= (uint64_t)sms * 1024;
-    const uint64_t threads = row ? k.outputs * k.group : (col_vec ? k.outputs / V : k.outputs);
-    const int grid = (int)std::max<uint64_t>(1, std::min<uint64_t>((uint64_t)sms * 8, (threads + 255) / 256));
-    if (dtype == F64) {
-        if (row_vec) gs_row_vec_kernel<double><<<grid, 256, 0, st>>>(k);
-        else if (row) gs_row_kernel<double><<<grid, 256, 0, st>>>(k);
-        else if (col_vec) gs_col_vec_kernel<double><<<grid, 256, 0, st>>>(k);
-        else gs_col_kernel<double><<<grid, 256, 0, st>>>(k);
-    } else {
-        if (row_vec) gs_row_vec_kernel<float><<<grid, 256, 0, st>>>(k);
-        else if (row) gs_row_kernel<float><<<grid, 256, 0, st>>>(k);
-        else if (col_vec) gs_col_vec_kernel<float><<<grid, 256, 0, st>>>(k);
-        else gs_col_kernel<float><<<grid, 256, 0, st>>>(k);
-    }
-    cudaError_t e = cudaGetLastError();
+    pl.f64 = dtype == F64;
+    gs_plan(sms, &pl);
+    if (pl.k.nseg > 1)
+        if (int s = get_scratch(st, (size_t)pl.k.nseg * pl.k.outputs * 2 * elem_size_t(dtype), &pl.k.part)) return s;
+    uint64_t launches = 0;
+    const cudaError_t e = gs_launch(pl, st, sms, &launches);
+    g_launches += launches;
     if (e != cudaSuccess) return cuda_fail(e, "kernel launch");
-    g_launches += 1;
     return ok();
 }
 
