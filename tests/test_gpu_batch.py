@@ -197,3 +197,42 @@ def test_recorded_costs(engine, orc, cuda):
     with B.Batch(probs) as bt:   # not recording: costs stay zero
         bt.launch()
         assert (bt.costs() == 0).all()
+
+
+@pytest.mark.parametrize("big", [0, 1, 24], ids=["tiny", "one-large", "several-large"])
+@pytest.mark.parametrize("select", ["heuristic", "learned"])
+def test_units_of_small_batches(engine, orc, cuda, select, big):
+    """The units follow the size of the launch (lanes per row, warps along q, bytes per unit):
+    contracted modes around every step of the rule, odd and even prefixes and rows, and problems
+    large enough to move the launch through the rule's range; variants and costs come back in
+    problem order.  Bar: two roundings per product, the merges' and the result's (4 x 2^-24 of
+    sum |a b|)."""
+    import torch
+    from ttv_gb300 import batch as B
+    g = torch.Generator(device=cuda)
+    g.manual_seed(big)
+    shapes = [([s, n, p], [3, 2, 1], 2)
+              for n in (1, 4, 7, 63, 64, 65, 129, 255, 512, 2000, 5000) for p, s in ((1, 33), (6, 5), (64, 3), (513, 2))]
+    shapes += [([700, 1500 + 4 * i], [1, 2], 1 + i % 2) for i in range(big)]
+    shapes += [([8, 512, 1024], [3, 2, 1], 2)] * min(big, 4)
+    probs, host = [], []
+    for na, pia, q in shapes:
+        N = int(np.prod(na))
+        a = torch.rand(N, generator=g, device=cuda) * 2 - 1
+        b = torch.rand(na[q - 1], generator=g, device=cuda) * 2 - 1
+        probs.append(B.Problem(q, na, pia, a, b, torch.full((N // na[q - 1],), float("nan"), device=cuda)))
+        host.append((na, pia, q))
+    if select == "learned":
+        B.load_cost_model()
+    with B.Batch(probs, select=B.SELECT_LEARNED if select == "learned" else B.SELECT_HEURISTIC,
+                 record_costs=True) as bt:
+        for _ in range(2):
+            reset(probs)
+            bt.launch()
+            check_all(orc, probs, host, tol=4 * 2.0 ** -24)
+        if select == "heuristic":
+            assert np.array_equal(bt.variants(), B.features(probs)[2])
+        cost = bt.costs()
+    assert B.batch_device_error() == 0
+    work = np.array([np.prod(na) for na, _, _ in host], float)
+    assert (cost > 0).all() and np.corrcoef(np.log(work), np.log(cost.astype(float)))[0, 1] > 0.5

@@ -54,7 +54,7 @@ struct BProb {
     uint64_t unit_begin;   // first unit of the problem in its executor's unit space
     uint64_t part_off;     // in BPair elements
     uint64_t tiles;        // column units: tiles per segment
-    uint64_t tpu;          // column units: tiles per unit
+    uint64_t tpu;          // column units: tiles per unit; row units: rounds of the lane groups
     uint64_t upseg;        // column units: units per segment
     IdxDiv pdiv;           // column units: output -> slice (division by P)
     IdxDiv tdiv;           // column units: unit -> segment (division by the units per segment)
@@ -102,10 +102,10 @@ constexpr size_t BRT_WARP_BYTES = (size_t)BRT_NS * (BRT_MAX_NQ * 4 + BRT_SLOT);
 constexpr size_t BRT_SMEM = 128 + BRT_WARPS * BRT_WARP_BYTES;
 // rows per lane of a tile: 32 R rows of n_q floats fill at most BRT_TILE_BYTES
 __host__ __device__ inline uint32_t brt_rows_per_lane(uint64_t nq) { return nq <= 16 ? 4u : (nq <= 32 ? 2u : 1u); }
-__host__ __device__ inline uint64_t brt_units(uint64_t nq, uint64_t S)
+__host__ __device__ inline uint64_t brt_units(uint64_t nq, uint64_t S, uint32_t tpu)
 {
     const uint64_t tiles = (S + 32 * brt_rows_per_lane(nq) - 1) / (32 * brt_rows_per_lane(nq));
-    return (tiles + BRT_TPU - 1) / BRT_TPU;
+    return (tiles + tpu - 1) / tpu;
 }
 
 constexpr int BMAX_F32 = BSTAGE_BYTES / 4;
@@ -143,12 +143,36 @@ __host__ __device__ inline void decode_variant(int kind, int v, uint64_t nq, int
 #define TLIBG_BATCH_UNIT_BYTES 131072
 #endif
 
+// How a batch is cut: bytes of A per work unit, tiles per staged unit, and the
+// longest chain of dependent round trips to HBM a unit may hold (0: as the
+// variant has it).
+struct BShape {
+    uint64_t unit_bytes;
+    uint32_t staged_tpu;
+    uint32_t trips;
+};
+
+// The unit's lanes per row or warps along q: the variant's, and more while the
+// unit's chain of loads is longer than the shape allows.  A trip is 4 rows of a
+// 16-byte column, 12 or 8 of a narrow one, 16 elements of a row's lane.
+__host__ __device__ inline uint64_t unit_trips(int kind, int group, int vec, uint64_t rows)
+{
+    const uint64_t per = kind == KIND_ROW ? 16 : (vec >= 4 ? 4 : (vec == 2 ? 8 : 12));
+    return (rows + per * group - 1) / (per * group);
+}
+__host__ __device__ inline int unit_group(int kind, int group, int vec, uint64_t nq, const BShape& sh)
+{
+    const int most = kind == KIND_ROW ? 32 : 8;
+    while (sh.trips != 0 && group < most && unit_trips(kind, group, vec, nq) > sh.trips) group *= 2;
+    return group;
+}
+
 // Row form: rounds of one row segment per lane group that make up a work unit.
-__host__ __device__ inline uint64_t rows_per_group(uint64_t seg_len, int group)
+__host__ __device__ inline uint64_t rows_per_group(uint64_t seg_len, int group, uint64_t unit_bytes)
 {
     const uint64_t gpc = BLOCK / group;
     const uint64_t per_round = gpc * seg_len * 4;
-    uint64_t r = (TLIBG_BATCH_UNIT_BYTES + per_round - 1) / per_round;
+    uint64_t r = (unit_bytes + per_round - 1) / per_round;
     return r < 1 ? 1 : (r > 256 ? 256 : r);
 }
 
@@ -161,27 +185,27 @@ __host__ __device__ inline uint64_t col_tile_outputs(int group, int vec)
 }
 
 // Column form: a unit is `tpu` consecutive tiles of one segment.
-__host__ __device__ inline uint64_t tiles_per_unit(uint64_t TO, uint64_t seg_len, uint64_t tiles)
+__host__ __device__ inline uint64_t tiles_per_unit(uint64_t TO, uint64_t seg_len, uint64_t tiles, uint64_t unit_bytes)
 {
-    uint64_t t = TLIBG_BATCH_UNIT_BYTES / (TO * seg_len * 4);
+    uint64_t t = unit_bytes / (TO * seg_len * 4);
     if (t < 1) t = 1;
     return t > tiles ? tiles : t;
 }
 
 __host__ __device__ inline uint64_t unit_count(int kind, int group, int vec, uint64_t P, uint64_t nq,
-                                               uint64_t S, uint32_t nseg, uint64_t* seg_len)
+                                               uint64_t S, uint32_t nseg, uint64_t unit_bytes, uint64_t* seg_len)
 {
     uint64_t sl = (nq + nseg - 1) / nseg;
     if (kind == KIND_ROW) sl = (sl + vec - 1) / vec * vec;
     *seg_len = sl;
     const uint64_t ns = (nq + sl - 1) / sl;
     if (kind == KIND_ROW) {
-        const uint64_t per_unit = (BLOCK / group) * rows_per_group(sl, group);
+        const uint64_t per_unit = (BLOCK / group) * rows_per_group(sl, group, unit_bytes);
         return (S * ns + per_unit - 1) / per_unit;
     }
     const uint64_t TO = col_tile_outputs(group, vec);
     const uint64_t tiles = (S * P + TO - 1) / TO;
-    const uint64_t tpu = tiles_per_unit(TO, sl, tiles);
+    const uint64_t tpu = tiles_per_unit(TO, sl, tiles, unit_bytes);
     return (tiles + tpu - 1) / tpu * ns;
 }
 
@@ -241,7 +265,7 @@ __global__ void batch_set_variant(BProb* __restrict__ pr, int n, int v)
 // --------------------------------------------------------------------------
 constexpr int PLAN_SUMS = 4;   // units of the three executor classes, split partials
 
-__global__ void __launch_bounds__(1024) batch_plan(BProb* __restrict__ pr, int n, BCtl* ctl)
+__global__ void __launch_bounds__(1024) batch_plan(BProb* __restrict__ pr, int n, BCtl* ctl, BShape sh)
 {
     __shared__ unsigned long long s_sum[PLAN_SUMS][32];
     __shared__ unsigned long long carry[PLAN_SUMS];
@@ -258,8 +282,9 @@ __global__ void __launch_bounds__(1024) batch_plan(BProb* __restrict__ pr, int n
             int group;
             uint32_t nseg;
             decode_variant(P.kind, P.variant, P.nq, &group, &nseg);
+            group = unit_group(P.kind, group, P.vec, P.nq, sh);
             uint64_t seg_len;
-            const uint64_t u = unit_count(P.kind, group, P.vec, P.P, P.nq, P.S, nseg, &seg_len);
+            const uint64_t u = unit_count(P.kind, group, P.vec, P.P, P.nq, P.S, nseg, sh.unit_bytes, &seg_len);
             nseg = (uint32_t)((P.nq + seg_len - 1) / seg_len);
             P.group = group;
             P.nseg = nseg;
@@ -270,17 +295,18 @@ __global__ void __launch_bounds__(1024) batch_plan(BProb* __restrict__ pr, int n
             if (P.kind == KIND_COL) {
                 const uint64_t TO = col_tile_outputs(group, P.vec);
                 P.tiles = (outputs + TO - 1) / TO;
-                P.tpu = tiles_per_unit(TO, seg_len, P.tiles);
+                P.tpu = tiles_per_unit(TO, seg_len, P.tiles, sh.unit_bytes);
                 P.upseg = (P.tiles + P.tpu - 1) / P.tpu;
                 P.pdiv = make_idx_div(P.P, outputs);
                 P.tdiv = make_idx_div(P.upseg, P.upseg * nseg);
             } else {
                 P.tiles = 0;
+                P.tpu = P.staged ? sh.staged_tpu : rows_per_group(seg_len, group, sh.unit_bytes);
                 P.sdiv = make_idx_div(nseg, P.S * nseg);
             }
             P.cls = P.staged ? CLS_STAGED : (P.kind == KIND_COL && P.vec <= 2 ? CLS_COL1 : CLS_GENERIC);
             if (P.staged) {
-                P.units = (uint32_t)brt_units(P.nq, P.S);
+                P.units = (uint32_t)brt_units(P.nq, P.S, sh.staged_tpu);
             } else {
                 P.units = (uint32_t)u;
                 x[3] = nseg > 1 ? (unsigned long long)nseg * outputs : 0ull;
@@ -409,7 +435,7 @@ __device__ __forceinline__ void row_unit(const BProb& P, uint64_t lu, int G, BPa
     const uint32_t lane = threadIdx.x & 31u, gl = lane & (uint32_t)(G - 1);
     const uint64_t gpc = BLOCK / G;
     const uint64_t items = P.S * P.nseg;
-    const uint64_t R = rows_per_group(P.seg_len, G);
+    const uint64_t R = P.tpu;
     constexpr int U = (int)sizeof(float) * V >= 16 ? 4 : 64 / ((int)sizeof(float) * V);
     constexpr int M = U / 2;
     if (P.nseg == 1 && P.nq % V == 0 && P.nq / V <= (uint64_t)G * M) {
@@ -906,8 +932,8 @@ __global__ void __launch_bounds__(BRT_THREADS) batch_rowtile(BProb* __restrict__
             const BProb& P = pr[iprob];
             const uint64_t R = brt_rows_per_lane(P.nq);
             const uint64_t tiles = (P.S + 32 * R - 1) / (32 * R);
-            it = (u - P.unit_begin) * BRT_TPU;
-            it_end = min(tiles, it + BRT_TPU);
+            it = (u - P.unit_begin) * P.tpu;
+            it_end = min(tiles, it + P.tpu);
         }
         return true;
     };
@@ -1082,6 +1108,27 @@ int heuristic_variant(int kind, uint64_t P, uint64_t nq, uint64_t S, int vec)
     return FIXED_RULE[kind == KIND_ROW ? 0 : 1][vi][shrt];
 }
 
+// Units of a batch whose variants the engine chose.  The launch cannot end
+// before its longest unit, so in a batch of a few hundred problems the units
+// shrink with the launch: the chain of loads of one unit (about TRIP_US a round
+// trip) to an eighth of the launch at full HBM rate, its bytes to a third of a
+// resident CTA's share.  Large batches keep the tuned units.  A unit of 512 rows
+// walked by one warp row is 128 round trips, all of a 64-problem launch: 120 us,
+// 64 with these units; 128 problems 175 -> 123 (139 with a quarter, 127 with a
+// sixteenth), 256: 215 -> 162, 512: 372 -> 341.
+BShape batch_shape(uint64_t bytes, int sms)
+{
+    constexpr double HBM_BYTES_PER_US = 6.5e6, TRIP_US = 0.9;
+    const double us = (double)bytes / HBM_BYTES_PER_US;
+    BShape sh{TLIBG_BATCH_UNIT_BYTES, BRT_TPU, 0};
+    const uint64_t share = bytes / ((uint64_t)sms * TLIBG_BATCH_MIN_CTAS * 3);
+    sh.unit_bytes = std::min<uint64_t>(TLIBG_BATCH_UNIT_BYTES, std::max<uint64_t>(16384, share));
+    sh.staged_tpu = (uint32_t)std::max<uint64_t>(1, sh.unit_bytes * BRT_TPU / TLIBG_BATCH_UNIT_BYTES);
+    const double trips = us / 8 / TRIP_US;
+    sh.trips = trips >= 128 ? 0u : (uint32_t)std::max(2.0, trips);
+    return sh;
+}
+
 }  // namespace
 }  // namespace tlibg
 
@@ -1101,6 +1148,8 @@ struct tlibg_batch {
     float* d_model = nullptr;
     float log2_count = 0.f;
     float log2_keep = 0.f;   // log2(1 - margin)
+    BShape shape{TLIBG_BATCH_UNIT_BYTES, BRT_TPU, 0};
+    std::vector<uint32_t> order;   // descriptor -> problem (longest units first)
     bool planned = false;          // the plan kernels ran for the current variants
     cudaStream_t side[2] = {nullptr, nullptr};      // the scalar-column and staged-row kernels' streams
     cudaEvent_t ev_fork = nullptr, ev_join[2] = {nullptr, nullptr};
@@ -1120,7 +1169,7 @@ int enqueue_plan(tlibg_batch* bt, cudaStream_t st)
         batch_set_variant<<<(bt->count + 255) / 256, 256, 0, st>>>(bt->d_prob, bt->count, bt->fixed_variant);
         ++n;
     }
-    batch_plan<<<1, 1024, 0, st>>>(bt->d_prob, bt->count, bt->d_ctl);
+    batch_plan<<<1, 1024, 0, st>>>(bt->d_prob, bt->count, bt->d_ctl, bt->shape);
     batch_fill_maps<<<(bt->count + 7) / 8, 256, 0, st>>>(bt->d_prob, bt->count, bt->d_map[0], bt->d_map[1],
                                                         bt->d_map[2]);
     n += 2;
@@ -1289,6 +1338,17 @@ int tlibg_batch_create(int dtype, const tlibg_problem* probs, size_t count, cons
     if (bt->select == TLIBG_SELECT_GIVEN && !have_given)
         return create_fail(bt, TLIBG_ERR_ARGUMENT, "tlibg_batch_create: TLIBG_SELECT_GIVEN needs variants");
 
+    // canonical views, and A's bytes for the shape of the units
+    std::vector<CanonView> views(count);
+    uint64_t total_bytes = 0;
+    for (size_t i = 0; i < count; ++i) {
+        const tlibg_problem& x = probs[i];
+        internal_analyse(x.q, x.p, x.a, x.na, x.wa, x.pia, x.b, x.nb, x.c, x.nc, x.wc, x.pic, &views[i]);
+        total_bytes += 4 * views[i].P * views[i].nq * views[i].S;
+    }
+    // forced and given variants run as they are (the tuner times them)
+    if (bt->select == TLIBG_SELECT_HEURISTIC || bt->select == TLIBG_SELECT_LEARNED) bt->shape = batch_shape(total_bytes, sms);
+
     // descriptors; unit map and partial scratch sized for the worst variant of each problem
     std::vector<BProb> hp(count);
     uint64_t total_units[NCLS] = {0, 0, 0}, max_part = 0;
@@ -1299,8 +1359,7 @@ int tlibg_batch_create(int dtype, const tlibg_problem* probs, size_t count, cons
             release(bt);
             return s;
         }
-        CanonView cn;
-        internal_analyse(x.q, x.p, x.a, x.na, x.wa, x.pia, x.b, x.nb, x.c, x.nc, x.wc, x.pic, &cn);
+        const CanonView& cn = views[i];
         BProb& b = hp[i];
         std::memset(&b, 0, sizeof(b));
         b.a = static_cast<const float*>(x.a);
@@ -1330,8 +1389,9 @@ int tlibg_batch_create(int dtype, const tlibg_problem* probs, size_t count, cons
             int g;
             uint32_t ns;
             decode_variant(b.kind, v, b.nq, &g, &ns);
+            g = unit_group(b.kind, g, b.vec, b.nq, bt->shape);
             uint64_t sl;
-            mu = std::max(mu, unit_count(b.kind, g, b.vec, b.P, b.nq, b.S, ns, &sl));
+            mu = std::max(mu, unit_count(b.kind, g, b.vec, b.P, b.nq, b.S, ns, bt->shape.unit_bytes, &sl));
             const uint64_t nsr = (b.nq + sl - 1) / sl;
             if (nsr > 1) mp = std::max(mp, nsr * b.S * b.P);
         }
@@ -1339,7 +1399,7 @@ int tlibg_batch_create(int dtype, const tlibg_problem* probs, size_t count, cons
         // decide), and in the staged class where that variant applies
         total_units[(b.kind == KIND_COL && b.vec <= 2) ? CLS_COL1 : CLS_GENERIC] += mu;
         max_part += mp;
-        if ((b.valid_mask >> VARIANT_STAGED) & 1u) total_units[CLS_STAGED] += brt_units(b.nq, b.S);
+        if ((b.valid_mask >> VARIANT_STAGED) & 1u) total_units[CLS_STAGED] += brt_units(b.nq, b.S, bt->shape.staged_tpu);
     }
     bt->slots[CLS_GENERIC] = exec_ctas_per_sm(bt->kahan, CLS_GENERIC);
     bt->slots[CLS_COL1] = exec_ctas_per_sm(bt->kahan, CLS_COL1);
@@ -1370,6 +1430,25 @@ int tlibg_batch_create(int dtype, const tlibg_problem* probs, size_t count, cons
         (!model.empty() && (e = internal_malloc((void**)&bt->d_model, MLP_PARAMS * sizeof(float))) != cudaSuccess)) {
         cudaGetLastError();
         return create_fail(bt, TLIBG_ERR_NOMEM, std::string("tlibg_batch_create: ") + cudaGetErrorString(e));
+    }
+    // Problems whose units hold the longest chains of loads go first in the queues
+    // (stable), so the short ones level the end of the launch.
+    bt->order.resize(count);
+    for (size_t i = 0; i < count; ++i) bt->order[i] = (uint32_t)i;
+    {
+        std::vector<uint64_t> chain(count);
+        for (size_t i = 0; i < count; ++i) {
+            const BProb& b = hp[i];
+            int g;
+            uint32_t ns;
+            decode_variant(b.kind, b.variant, b.nq, &g, &ns);
+            g = unit_group(b.kind, g, b.vec, b.nq, bt->shape);
+            chain[i] = unit_trips(b.kind, g, b.vec, (b.nq + ns - 1) / ns);
+        }
+        std::stable_sort(bt->order.begin(), bt->order.end(), [&](uint32_t x, uint32_t y) { return chain[x] > chain[y]; });
+        std::vector<BProb> sorted(count);
+        for (size_t i = 0; i < count; ++i) sorted[i] = hp[bt->order[i]];
+        hp.swap(sorted);
     }
     cudaMemcpyAsync(bt->d_prob, hp.data(), count * sizeof(BProb), cudaMemcpyHostToDevice, st);
     BCtl hctl{};
@@ -1468,7 +1547,7 @@ int tlibg_batch_variants(tlibg_batch* bt, int* out, void* stream)
     cudaError_t e = cudaMemcpyAsync(hp.data(), bt->d_prob, bt->count * sizeof(BProb), cudaMemcpyDeviceToHost, st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
     if (e != cudaSuccess) return internal_cuda_fail(e, "tlibg_batch_variants");
-    for (int i = 0; i < bt->count; ++i) out[i] = hp[i].variant;
+    for (int i = 0; i < bt->count; ++i) out[bt->order[i]] = hp[i].variant;
     return internal_ok();
 }
 
@@ -1483,7 +1562,7 @@ int tlibg_batch_costs(tlibg_batch* bt, uint64_t* cycles, void* stream)
     // SM cycles: a unit's CTA (or, staged, warp) cycles over the CTAs (warps) resident per SM
     for (int i = 0; i < bt->count; ++i) {
         const uint64_t sl = (uint64_t)bt->slots[hp[i].cls];
-        cycles[i] = (hp[i].cycles + sl / 2) / sl;
+        cycles[bt->order[i]] = (hp[i].cycles + sl / 2) / sl;
     }
     return internal_ok();
 }
