@@ -131,6 +131,32 @@ int tlibg_ttv_ex(int dtype, size_t q, size_t p,
                  void* c, const size_t* nc, const size_t* wc, const size_t* pic,
                  const tlibg_options* opt, void* stream);
 
+/* Packed forms, for language bindings whose foreign calls cost by the argument:
+ * one array of 64-bit words, TLIBG_PACKED_WORDS of fixed meaning (the indices
+ * below; TLIBG_PACKED_BYTES: the sizes in bytes of the buffers behind a, b and
+ * c, three words, UINT64_MAX where unknown; a smaller buffer than its layout
+ * addresses is TLIBG_ERR_ARGUMENT; TLIBG_PACKED_OPTIONS: tlibg_options' six
+ * fields in order), then the call's arrays back to back:
+ *   tlibg_ttv_packed            na wa pia (p each) nb (1) nc wc pic (p-1 each)
+ *   tlibg_ttv_packed_rowmajor   na wa (p each) nb (1); layout (p, .., 1), C's
+ *                               shape, dense strides and layout derived from it
+ *   tlibg_ttv_strided_packed    as the first, then wb (1); sizes in elements;
+ *                               options unused
+ *   tlibg_ttvs_packed_rowmajor  na wa (p each), the vectors' lengths and their
+ *                               addresses (p-1 each); layout (p, .., 1); b,
+ *                               sizes and options unused
+ * Checks, messages and results are those of tlibg_ttv_ex, tlibg_ttv_strided
+ * and tlibg_ttvs. */
+enum {
+    TLIBG_PACKED_DTYPE = 0, TLIBG_PACKED_Q = 1, TLIBG_PACKED_P = 2, TLIBG_PACKED_A = 3, TLIBG_PACKED_B = 4,
+    TLIBG_PACKED_C = 5, TLIBG_PACKED_BYTES = 6, TLIBG_PACKED_STREAM = 9, TLIBG_PACKED_OPTIONS = 10,
+    TLIBG_PACKED_WORDS = 16
+};
+int tlibg_ttv_packed(const uint64_t* words);
+int tlibg_ttv_packed_rowmajor(const uint64_t* words);
+int tlibg_ttv_strided_packed(const uint64_t* words);
+int tlibg_ttvs_packed_rowmajor(const uint64_t* words);
+
 /* Extension (no reference counterpart): the same contraction on DEVICE
  * pointers with the natural meaning of every stride, for sliced, padded or
  * transposed views -- A's element (i_1..i_p) at a[sum_r i_r wa[r]] (zero-based

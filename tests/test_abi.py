@@ -430,3 +430,140 @@ def test_strided_extension_checks(engine):
     assert st in (engine.ERR_CUDA, engine.ERR_ARGUMENT, engine.OK)
     if st == engine.ERR_ARGUMENT:
         assert "device-accessible" in msg
+
+
+def _packed(engine, dtype, q, p, ptrs, sizes, words, opts=(0, -1, 0, 0, 0, 0)):
+    import struct
+    return struct.pack(f"=10Q6q{len(words)}Q", dtype, q, p, *ptrs, *sizes, 0, *opts, *words)
+
+
+def _outcome(engine, st):
+    msg = engine._last_error()
+    # past every host check: no device, or (with one) the stand-in pointers refused
+    if st in (engine.ERR_CUDA, engine.OK) or (st == engine.ERR_ARGUMENT and "device-accessible" in msg):
+        return "passed the checks"
+    return st, msg
+
+
+def _mutated(rng, p):
+    """Metadata of an order-p call, valid or with one or two entries spoiled."""
+    na = [int(x) for x in rng.integers(1, 6, p)]
+    pia = [int(x) + 1 for x in rng.permutation(p)]
+    q = int(rng.integers(1, p + 1))
+    wa, acc = [0] * p, 1
+    for m in pia:
+        wa[m - 1], acc = acc, acc * na[m - 1]
+    nc = [n for m, n in enumerate(na) if m != q - 1]
+    pic = [m - (m > q) for m in pia if m != q]
+    wc, acc = [0] * (p - 1), 1
+    for m in pic:
+        wc[m - 1], acc = acc, acc * nc[m - 1]
+    nb = [na[q - 1]]
+    lists = [na, wa, pia, nb, nc, wc, pic]
+    for _ in range(int(rng.integers(0, 3))):
+        v = lists[int(rng.integers(0, 7))]
+        v[int(rng.integers(0, len(v)))] = int(rng.choice([0, 1, 2, 3, 7, 1000, 2 ** 33, 2 ** 63]))
+    if rng.random() < 0.1:
+        q = int(rng.choice([0, p + 1, 2 ** 63]))
+    return q, lists
+
+
+def test_packed_calls_answer_like_the_general_ones(engine):
+    """The packed forms give the general calls' status and message on 4000 random calls, valid
+    and spoiled, at every dtype, through the dense and the strided entry points."""
+    lib = engine.library()
+    rng = np.random.default_rng(20)
+    big = 2 ** 64 - 1
+    seen = set()
+    for _ in range(4000):
+        p = int(rng.integers(2, 6))
+        q, lists = _mutated(rng, p)
+        na, wa, pia, nb, nc, wc, pic = lists
+        dt = int(rng.integers(0, 4))
+        ptrs = [int(x) for x in rng.choice([0, 16, 16, 16, 18, 4096], 3)]
+        flat = [x for v in lists for x in v]
+        general = _outcome(engine, _call(engine, dt, q, p, *lists, *ptrs))
+        packed = _outcome(engine, lib.tlibg_ttv_packed(_packed(engine, dt, q, p, ptrs, (big,) * 3, flat)))
+        assert packed == general, (q, lists, dt, ptrs)
+        seen.add(general)
+        wb = int(rng.choice([0, 1, 3]))
+        keep = [engine._sizes(v) for v in lists]
+        st = lib.tlibg_ttv_strided(dt, q, p, ptrs[0], *[engine._p(k) for k in keep[:3]], ptrs[1], engine._p(keep[3]),
+                                   wb, ptrs[2], *[engine._p(k) for k in keep[4:]], None)
+        general = _outcome(engine, st)
+        packed = _outcome(engine, lib.tlibg_ttv_strided_packed(
+            _packed(engine, dt, q, p, ptrs, (big,) * 3, flat + [wb])))
+        assert packed == general, (q, lists, dt, ptrs, wb)
+    assert len(seen) > 12
+
+
+def test_packed_calls_check_buffer_sizes(engine):
+    """Sizes are compared with what the layouts address, after the metadata checks; strides whose
+    span passes 64 bits count as too large, not as small."""
+    lib = engine.library()
+    q, p, lists = 1, 3, [[4, 5, 6], [1, 4, 20], [1, 2, 3], [4], [5, 6], [1, 5], [1, 2]]
+    flat = [x for v in lists for x in v]
+    for dt, (ea, et) in ((0, (4, 4)), (1, (8, 8)), (2, (2, 4))):
+        need = [120 * ea, 4 * et, 30 * et]
+        for i in range(3):
+            short = list(need)
+            short[i] -= 1
+            st = lib.tlibg_ttv_packed(_packed(engine, dt, q, p, (16, 32, 48), short, flat))
+            assert (st, engine._last_error()) == (engine.ERR_ARGUMENT, f"tlibg: buffer {'abc'[i]} holds {short[i]} "
+                                                                       f"bytes, its layout addresses {need[i]}")
+        assert _outcome(engine, lib.tlibg_ttv_packed(
+            _packed(engine, dt, q, p, (16, 32, 48), need, flat))) == "passed the checks"
+        # C's strides do not matter to the reference here (q fastest), but the buffer check counts them
+        lists2 = [list(v) for v in lists]
+        lists2[5] = [2 ** 62, 2 ** 63]
+        st = lib.tlibg_ttv_packed(_packed(engine, dt, q, p, (16, 32, 48), need, [x for v in lists2 for x in v]))
+        assert st == engine.ERR_ARGUMENT and "buffer c holds" in engine._last_error()
+
+
+def test_packed_rowmajor_derives_the_metadata(engine):
+    """tlibg_ttv_packed_rowmajor answers as the packed call with the metadata helpers' layout."""
+    lib = engine.library()
+    rng = np.random.default_rng(5)
+    for _ in range(400):
+        p = int(rng.integers(2, 7))
+        na = [int(x) for x in rng.integers(1, 5, p)]
+        q = int(rng.integers(1, p + 1))
+        pia = list(range(p, 0, -1))
+        wa = [int(np.prod(na[r + 1:])) for r in range(p)]
+        if rng.random() < 0.2:
+            wa[int(rng.integers(0, p))] = int(rng.integers(0, 9))
+        nb = na[q - 1] + (1 if rng.random() < 0.1 else 0)
+        nc, pic = engine.output_shape(na, q), engine.output_layout(pia, q)
+        wc = engine.strides(nc, pic)
+        need = [4 * (1 + sum((n - 1) * w for n, w in zip(na, wa))), 4 * nb, 4 * int(np.prod(nc))]
+        if rng.random() < 0.2:
+            need[int(rng.integers(0, 3))] -= 4
+        a = _outcome(engine, lib.tlibg_ttv_packed(
+            _packed(engine, 0, q, p, (16, 32, 48), need, [*na, *wa, *pia, nb, *nc, *wc, *pic])))
+        b = _outcome(engine, lib.tlibg_ttv_packed_rowmajor(
+            _packed(engine, 0, q, p, (16, 32, 48), need, [*na, *wa, nb])))
+        assert a == b, (na, q, wa, nb)
+
+
+def test_python_calls_keep_their_answers(engine):
+    """Arguments the packed form does not take (None, floats, longer lists, raw addresses, empty
+    tensors) go through the general one: the same errors as before."""
+    import torch
+    t = torch.zeros(120)
+    b, c = torch.zeros(4), torch.zeros(30)
+    meta = ([4, 5, 6], [1, 4, 20], [1, 2, 3])
+    out = ([5, 6], [1, 5], [1, 2])
+    with pytest.raises(engine.TTVError, match="pointer to input tensor shape vector na should not be zero"):
+        engine.ttv(1, 3, 16, None, *meta[1:], 32, [4], 48, *out)
+    with pytest.raises((engine.DeviceError, engine.TTVError), match="CUDA|device"):
+        engine.ttv(1, 3, t, [4.0, 5.0, 6.0], *meta[1:], b, [4], c, *out)
+    with pytest.raises((engine.DeviceError, engine.TTVError), match="CUDA|device"):
+        engine.ttv(1, 3, t, [4, 5, 6, 9], *meta[1:], b, (4,), c, *out)
+    with pytest.raises(engine.TTVError, match="shape vector of A is not valid"):
+        engine.ttv(1, 3, torch.zeros(0), [4, 0, 6], *meta[1:], b, [4], c, *out)
+    with pytest.raises(engine.TTVError, match="contraction mode should be greater zero"):
+        engine.ttv(-1, 3, t, *meta, b, [4], c, *out)
+    with pytest.raises(TypeError):
+        engine.ttv(1, 3, t, *meta, b, [4], c, *out, no_such_option=1)
+    with pytest.raises(engine.TTVError, match="contraction dimension of A and B are not equal"):
+        engine.ttv_array(2, torch.zeros(4, 5), torch.zeros(4))

@@ -23,6 +23,7 @@ from __future__ import annotations
 
 import ctypes as C
 import os
+import struct
 
 __all__ = [
     "TTVError", "UnsupportedError", "ttv", "ttv_ex", "ttv_host", "ttv_array", "ttvs", "plan",
@@ -123,6 +124,11 @@ def library() -> C.CDLL:
         L.tlibg_plan_hint.restype = C.c_int
         L.tlibg_plan_hint.argtypes = [C.c_int, C.c_uint64, C.c_uint64, C.c_uint64,
                                       C.POINTER(Options)]
+        for name in ("tlibg_ttv_packed", "tlibg_ttv_packed_rowmajor", "tlibg_ttv_strided_packed",
+                     "tlibg_ttvs_packed_rowmajor"):
+            f = getattr(L, name)
+            f.restype = C.c_int
+            f.argtypes = [C.c_char_p]
         L.tlibg_version.restype = C.c_char_p
         _lib = L
     return _lib
@@ -165,14 +171,24 @@ def _ptr(x):
     return x.data_ptr()
 
 
+_raw_stream = None   # torch's current stream of the current device, as an address
+
+
 def _stream_handle(stream):
+    global _raw_stream
     if stream is None:
         try:
             import torch
-            if torch.cuda.is_available():
-                return torch.cuda.current_stream().cuda_stream
         except ImportError:
-            pass
+            return None
+        if torch.cuda.is_initialized():
+            if _raw_stream is None:
+                get, dev = (getattr(torch._C, n, None) for n in ("_cuda_getCurrentRawStream", "_cuda_getDevice"))
+                _raw_stream = (lambda: get(dev())) if get and dev else \
+                    (lambda: torch.cuda.current_stream().cuda_stream)
+            return _raw_stream()
+        if torch.cuda.is_available():
+            return torch.cuda.current_stream().cuda_stream
         return None
     if isinstance(stream, int):
         return stream
@@ -181,6 +197,30 @@ def _stream_handle(stream):
 
 def _options(accumulate=ACC_COMPENSATED, kind=-1, group=0, vec=0, split=0, sync=False):
     return Options(int(accumulate), int(kind), int(group), int(vec), int(split), int(bool(sync)))
+
+
+# --------------------------------------------------------------------------
+# packed calls: one array of words (tlibg.h, "Packed forms") instead of a
+# dozen converted arguments and seven ctypes arrays: 59 -> 12 us a small call
+# --------------------------------------------------------------------------
+_DEFAULT_OPTIONS = (ACC_COMPENSATED, -1, 0, 0, 0, 0)
+_packers = {}
+_UNPLAIN = (TypeError, AttributeError, struct.error)   # arguments only the general form takes
+
+
+def _pack(dtype, q, p, a, b, c, sizes, stream, opts, *words):
+    """The call's words, or None where a tensor is empty (a null address)."""
+    pa, pb, pc = a.data_ptr(), b.data_ptr(), c.data_ptr()
+    if not (pa and pb and pc):
+        return None
+    n = len(words)
+    pack = _packers.get(n)
+    if pack is None:
+        pack = _packers[n] = struct.Struct(f"=10Q6q{n}Q").pack
+    if opts:
+        o = _options(**opts)
+        opts = [getattr(o, f) for f, _ in Options._fields_]
+    return pack(dtype, q, p, pa, pb, pc, *sizes, _stream_handle(stream) or 0, *(opts or _DEFAULT_OPTIONS), *words)
 
 
 # --------------------------------------------------------------------------
@@ -198,6 +238,16 @@ def ttv(q, p, a, na, wa, pia, b, nb, c, nc, wc, pic, *, dtype=None, stream=None,
     """
     if dtype is None:
         dtype = _dtype_of(a)
+    try:
+        words = None
+        if len(na) == len(wa) == len(pia) == p and len(nc) == len(wc) == len(pic) == p - 1 and len(nb) == 1:
+            words = _pack(dtype, q, p, a, b, c, (a.nbytes, b.nbytes, c.nbytes), stream, opts,
+                          *na, *wa, *pia, *nb, *nc, *wc, *pic)
+    except _UNPLAIN:
+        words = None
+    if words is not None:
+        _raise(library().tlibg_ttv_packed(words))
+        return c
     keep = [_sizes(v) for v in (na, wa, pia, nb, nc, wc, pic)]
     _check_buffers(dtype, q, p, keep, a, b, c)
     o = _options(**opts)
@@ -252,6 +302,17 @@ def ttv_strided(q, p, a, na, wa, pia, b, nb, c, nc, wc, pic, *, wb=1, dtype=None
     address."""
     if dtype is None:
         dtype = _dtype_of(a)
+    try:
+        words = None
+        if len(na) == len(wa) == len(pia) == p and len(nc) == len(wc) == len(pic) == p - 1 and len(nb) == 1:
+            # elements from each tensor's first element to the end of its storage (views too)
+            have = [t.untyped_storage().nbytes() // t.element_size() - t.storage_offset() for t in (a, b, c)]
+            words = _pack(dtype, q, p, a, b, c, have, stream, None, *na, *wa, *pia, *nb, *nc, *wc, *pic, wb)
+    except _UNPLAIN:
+        words = None
+    if words is not None:
+        _raise(library().tlibg_ttv_strided_packed(words))
+        return c
     keep = [_sizes(v) for v in (na, wa, pia, nb, nc, wc, pic)]
     need = {"a": _addressed(keep[0][:p], keep[1][:p]),
             "b": (int(keep[3][0]) - 1) * int(wb) + 1 if len(keep[3]) and int(keep[3][0]) else 0,
@@ -287,8 +348,8 @@ def ttv_view(q, A, b, out=None, *, stream=None):
         out = torch.empty(shape_c, dtype=A.dtype, device=A.device)
     wc = list(out.stride())
     # layouts that pass the reference's monotonic-stride check: modes by increasing stride
-    pia = [m + 1 for m in sorted(range(p), key=lambda m: (wa[m], m))]
-    pic = [m + 1 for m in sorted(range(p - 1), key=lambda m: (wc[m], m))] or [1]
+    pia = [m + 1 for m in sorted(range(p), key=wa.__getitem__)]
+    pic = [m + 1 for m in sorted(range(p - 1), key=wc.__getitem__)] or [1]
     return ttv_strided(q, p, A, na, wa, pia, b, [int(b.shape[0])], out, shape_c or [1], wc or [1], pic,
                        wb=int(b.stride(0)), stream=stream)
 
@@ -317,13 +378,22 @@ def _host_ptr(x):
     return x.data_ptr()
 
 
+_dtypes = {}   # element type objects already mapped
+
+
 def _dtype_of(a):
-    name = str(getattr(a, "dtype", "float32"))
-    if "float64" in name or name.endswith("double"):
-        return F64
-    if "bfloat16" in name or "uint16" in name:
-        return BF16A
-    return F32
+    dt = getattr(a, "dtype", "float32")
+    code = _dtypes.get(dt)
+    if code is None:
+        name = str(dt)
+        if "float64" in name or name.endswith("double"):
+            code = F64
+        elif "bfloat16" in name or "uint16" in name:
+            code = BF16A
+        else:
+            code = F32
+        _dtypes[dt] = code
+    return code
 
 
 def plan(q, na, pia, dtype=F32, **opts):
@@ -420,15 +490,25 @@ def ttv_array(q, A, b, *, out=None, stream=None, **opts):
     if not A.is_contiguous():
         A = A.contiguous()
     na = list(A.shape)
+    cdt = torch.float32 if A.dtype == torch.bfloat16 else A.dtype
+    dt = BF16A if A.dtype == torch.bfloat16 else (F64 if A.dtype == torch.float64 else F32)
+    if p > 1 and q > 0 and 0 not in na:
+        c = torch.empty(na[:q - 1] + na[q:], dtype=cdt, device=A.device) if out is None else out
+        try:
+            words = _pack(dt, q, p, A, b, c, (A.nbytes, b.nbytes, c.nbytes), stream, opts, *na, *A.stride(),
+                          b.shape[0])
+        except _UNPLAIN:
+            words = None
+        if words is not None:
+            _raise(library().tlibg_ttv_packed_rowmajor(words))
+            return c
     pia = list(range(p, 0, -1))
     wa = [s for s in A.stride()]
     nc = output_shape(na, q)
     pic = output_layout(pia, q)
     wc = strides(nc, pic)
-    cdt = torch.float32 if A.dtype == torch.bfloat16 else A.dtype
     if out is None:
         out = torch.empty(nc, dtype=cdt, device=A.device)
-    dt = BF16A if A.dtype == torch.bfloat16 else (F64 if A.dtype == torch.float64 else F32)
     a_ptr = A.view(torch.int16) if dt == BF16A else A
     ttv(q, p, a_ptr, na, wa, pia, b, [b.shape[0]], out, nc, wc, pic, dtype=dt, stream=stream,
         **opts)
@@ -492,11 +572,21 @@ def _ttvs_fused(q, A, bs, stream):
         A = A.contiguous()
     dt = BF16A if A.dtype == torch.bfloat16 else (F64 if A.dtype == torch.float64 else F32)
     vdt = torch.float64 if dt == F64 else torch.float32
-    vecs = [bj.to(device=A.device, dtype=vdt).contiguous() for bj in bs]
+    dev = A.device
+    vecs = [bj if bj.dtype == vdt and bj.device == dev and bj.is_contiguous() else
+            bj.to(device=dev, dtype=vdt).contiguous() for bj in bs]
     na = list(A.shape)
-    pia = list(range(p, 0, -1))
     wa = list(A.stride())
-    out = torch.empty(na[q - 1], dtype=vdt, device=A.device)
+    out = torch.empty(na[q - 1], dtype=vdt, device=dev)
+    try:
+        words = _pack(dt, q, p, A, A, out, (0, 0, 0), stream, None, *na, *wa, *[v.shape[0] for v in vecs],
+                      *[v.data_ptr() for v in vecs])
+    except _UNPLAIN:
+        words = None
+    if words is not None:
+        _raise(library().tlibg_ttvs_packed_rowmajor(words))
+        return out
+    pia = list(range(p, 0, -1))
     keep = [_sizes(v) for v in (na, wa, pia, [int(v.shape[0]) for v in vecs])]
     ptrs = (_vp * len(vecs))(*[v.data_ptr() for v in vecs])
     a_ptr = A.view(torch.int16) if dt == BF16A else A

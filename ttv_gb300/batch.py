@@ -16,7 +16,7 @@ import os
 
 import numpy as np
 
-from . import F32, _check_buffers, _last_error, _options, _p, _raise, _sizes, library, \
+from . import F32, _check_buffers, _last_error, _options, _p, _raise, _sizes, _stream_handle, library, \
     output_layout, output_shape, strides
 
 SELECT_HEURISTIC, SELECT_LEARNED, SELECT_FIXED, SELECT_GIVEN = 0, 1, 2, 3
@@ -79,8 +79,9 @@ def _lib():
 def _stream(stream):
     if stream is None:
         import torch
-        return torch.cuda.current_stream().cuda_stream
-    return stream if isinstance(stream, int) else stream.cuda_stream
+        if not torch.cuda.is_initialized():
+            return torch.cuda.current_stream().cuda_stream
+    return _stream_handle(stream)
 
 
 class Problem:

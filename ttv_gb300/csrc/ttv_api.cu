@@ -919,14 +919,48 @@ int check_elem_align(int dtype, const void* a, const void* b, const void* c)
     return TLIBG_OK;
 }
 
+// Elements a tensor with extents n and strides w spans (2^62 and more: 2^62).
+uint64_t addressed(const size_t* n, const size_t* w, size_t p)
+{
+    constexpr uint64_t MOST = uint64_t(1) << 62;
+    uint64_t last = 0;
+    for (size_t r = 0; r < p; ++r)
+        if (n[r] == 0) return 0;
+    for (size_t r = 0; r < p; ++r) {
+        uint64_t t;
+        if (mul_overflows(n[r] - 1, w[r], &t) || t >= MOST || (last += t) >= MOST) return MOST;
+    }
+    return last + 1;
+}
+
+// Buffers of known size (have[0..2]: a, b, c, in bytes or in elements) must hold what their layouts address; the kernels trust the
+// metadata as the reference does.
+int check_sizes(int dtype, const uint64_t* have, bool in_bytes, const uint64_t* need)
+{
+    const uint64_t es[3] = {elem_size_a(dtype), elem_size_t(dtype), elem_size_t(dtype)};
+    for (int i = 0; i < 3; ++i) {
+        if (have[i] == UINT64_MAX || (in_bytes ? have[i] / es[i] : have[i]) >= need[i]) continue;   // unknown, or enough
+        std::string m = std::string("tlibg: buffer ") + "abc"[i] + " holds " + std::to_string(have[i]);
+        m += in_bytes ? " bytes, its layout addresses " + std::to_string(need[i] * es[i])
+                      : " elements, its strides address " + std::to_string(need[i]);
+        return fail(TLIBG_ERR_ARGUMENT, m);
+    }
+    return TLIBG_OK;
+}
+
 int run_device(int dtype, size_t q, size_t p, const void* a, const size_t* na, const size_t* wa,
                const size_t* pia, const void* b, const size_t* nb, void* c, const size_t* nc,
-               const size_t* wc, const size_t* pic, const tlibg_options* opt, cudaStream_t stream)
+               const size_t* wc, const size_t* pic, const tlibg_options* opt, cudaStream_t stream,
+               const uint64_t* bytes = nullptr)
 {
     NvtxRange nvtx("tlibg_ttv");
     Canon cn;
     int st = analyse(q, p, a, na, wa, pia, b, nb, c, nc, wc, pic, &cn);
     if (st) return st;
+    if (bytes) {
+        const uint64_t need[3] = {addressed(na, wa, p), nb[0], addressed(nc, wc, p - 1)};
+        if ((st = check_sizes(dtype, bytes, true, need))) return st;
+    }
     st = check_elem_align(dtype, a, b, c);
     if (st) return st;
     DevInfo d = dev_info();
@@ -991,6 +1025,45 @@ int tlibg_ttv_ex(int dtype, size_t q, size_t p, const void* a, const size_t* na,
         return fail(TLIBG_ERR_ARGUMENT, "tlibg: unknown element type");
     return run_device(dtype, q, p, a, na, wa, pia, b, nb, c, nc, wc, pic, opt,
                       static_cast<cudaStream_t>(stream));
+}
+
+int tlibg_ttv_packed(const uint64_t* w)
+{
+    static_assert(sizeof(size_t) == sizeof(uint64_t), "packed words are size_t");
+    const int dtype = (int)w[TLIBG_PACKED_DTYPE];
+    const size_t q = w[TLIBG_PACKED_Q], p = w[TLIBG_PACKED_P];
+    if (dtype != F32 && dtype != F64 && dtype != BF16A)
+        return fail(TLIBG_ERR_ARGUMENT, "tlibg: unknown element type");
+    if (p == 0) return fail(TLIBG_ERR_ARGUMENT, MSG[1]);
+    auto ptr = [&](int i) { return reinterpret_cast<void*>(w[i]); };
+    const tlibg_options opt{(int)w[TLIBG_PACKED_OPTIONS],     (int)w[TLIBG_PACKED_OPTIONS + 1],
+                            (int)w[TLIBG_PACKED_OPTIONS + 2], (int)w[TLIBG_PACKED_OPTIONS + 3],
+                            (int)w[TLIBG_PACKED_OPTIONS + 4], (int)w[TLIBG_PACKED_OPTIONS + 5]};
+    const size_t* na = reinterpret_cast<const size_t*>(w + TLIBG_PACKED_WORDS);
+    const size_t *wa = na + p, *pia = wa + p, *nb = pia + p, *nc = nb + 1, *wc = nc + (p - 1), *pic = wc + (p - 1);
+    return run_device(dtype, q, p, ptr(TLIBG_PACKED_A), na, wa, pia, ptr(TLIBG_PACKED_B), nb, ptr(TLIBG_PACKED_C), nc,
+                      wc, pic, &opt, static_cast<cudaStream_t>(ptr(TLIBG_PACKED_STREAM)), w + TLIBG_PACKED_BYTES);
+}
+
+int tlibg_ttv_packed_rowmajor(const uint64_t* w)
+{
+    // the last-order layout and C's metadata, then the call above
+    const size_t q = w[TLIBG_PACKED_Q], p = w[TLIBG_PACKED_P];
+    if (p < 2 || p > 64 || q == 0 || q > p)
+        return fail(TLIBG_ERR_ARGUMENT, "tlibg_ttv_packed_rowmajor: needs an order of 2 to 64 and a mode of it");
+    uint64_t v[TLIBG_PACKED_WORDS + 6 * 64];
+    std::memcpy(v, w, TLIBG_PACKED_WORDS * sizeof(uint64_t));
+    size_t* na = reinterpret_cast<size_t*>(v + TLIBG_PACKED_WORDS);
+    size_t *wa = na + p, *pia = wa + p, *nb = pia + p, *nc = nb + 1, *wc = nc + (p - 1), *pic = wc + (p - 1);
+    std::memcpy(na, w + TLIBG_PACKED_WORDS, 2 * p * sizeof(uint64_t));
+    nb[0] = w[TLIBG_PACKED_WORDS + 2 * p];
+    for (size_t r = 0; r < p; ++r) pia[r] = p - r;
+    for (size_t r = 0, o = 0; r < p; ++r)
+        if (r != q - 1) nc[o++] = na[r];
+    for (size_t r = 0, o = 0; r < p; ++r)
+        if (pia[r] != q) pic[o++] = pia[r] > q ? pia[r] - 1 : pia[r];
+    dense_strides(nc, pic, p - 1, wc);
+    return tlibg_ttv_packed(v);
 }
 
 int tlibg_validate(size_t q, size_t p, const size_t* na, const size_t* wa, const size_t* pia,
@@ -1148,6 +1221,21 @@ int tlibg_ttv_strided(int dtype, size_t q, size_t p, const void* a, const size_t
     return ok();
 }
 
+int tlibg_ttv_strided_packed(const uint64_t* w)
+{
+    const int dtype = (int)w[TLIBG_PACKED_DTYPE];
+    const size_t q = w[TLIBG_PACKED_Q], p = w[TLIBG_PACKED_P];
+    if (p == 0) return fail(TLIBG_ERR_ARGUMENT, MSG[1]);
+    auto ptr = [&](int i) { return reinterpret_cast<void*>(w[i]); };
+    const size_t* na = reinterpret_cast<const size_t*>(w + TLIBG_PACKED_WORDS);
+    const size_t *wa = na + p, *pia = wa + p, *nb = pia + p, *nc = nb + 1, *wc = nc + (p - 1), *pic = wc + (p - 1),
+                 *wb = pic + (p - 1);
+    const uint64_t need[3] = {addressed(na, wa, p), addressed(nb, wb, 1), p > 1 ? addressed(nc, wc, p - 1) : 0};
+    if (int st = check_sizes(dtype, w + TLIBG_PACKED_BYTES, false, need)) return st;
+    return tlibg_ttv_strided(dtype, q, p, ptr(TLIBG_PACKED_A), na, wa, pia, ptr(TLIBG_PACKED_B), nb, wb[0],
+                             ptr(TLIBG_PACKED_C), nc, wc, pic, ptr(TLIBG_PACKED_STREAM));
+}
+
 // ---------------------------------------------------------------------------
 // host-buffer path: chunked copies overlapped with the kernels
 // ---------------------------------------------------------------------------
@@ -1200,6 +1288,7 @@ int tlibg_ttv_host(int dtype, size_t q, size_t p, const void* a, const size_t* n
     const uint64_t nchunks = cdiv(cn.S, spc);
 
     struct HostCtx {
+        unsigned int* err = nullptr;   // page-locked: the device error word as the call's kernels left it
         cudaStream_t comp = nullptr, copy = nullptr;
         cudaEvent_t ev[2] = {nullptr, nullptr};
         cudaEvent_t done[2] = {nullptr, nullptr};
@@ -1224,7 +1313,25 @@ int tlibg_ttv_host(int dtype, size_t q, size_t p, const void* a, const size_t* n
             cudaEventCreateWithFlags(&hc.ev[i], cudaEventDisableTiming);
             cudaEventCreateWithFlags(&hc.done[i], cudaEventDisableTiming);
         }
+        if (cudaHostAlloc((void**)&hc.err, sizeof(*hc.err), cudaHostAllocDefault) != cudaSuccess) {
+            cudaGetLastError();
+            hc.err = nullptr;
+        }
     }
+    // End of a call: the error word follows the kernels on the stream, so one wait
+    // covers both (two synchronous copies of the word took 16 us of a 384 us call);
+    // it is cleared only when set.
+    auto finish = [&]() -> int {
+        if (hc.err && copy_device_error(hc.err, hc.comp) != cudaSuccess) {
+            cudaGetLastError();
+            *hc.err = 1u;   // unknown: ask the device below
+        }
+        const cudaError_t ee = cudaStreamSynchronize(hc.comp);
+        if (ee != cudaSuccess) return cuda_fail(ee, "stream synchronize");
+        if ((!hc.err || *hc.err) && read_and_clear_device_error())
+            return fail(TLIBG_ERR_TIMEOUT, "tlibg: a bounded device wait expired; results are invalid");
+        return ok();
+    };
     const size_t need_a = (size_t)(spc * panel * ea) + 32;   // + the 16-byte cover of a chunk
     const size_t need_b = (size_t)(cn.nq * et);
     const size_t need_c = (size_t)(cn.S * cn.P * et);
@@ -1307,10 +1414,7 @@ int tlibg_ttv_host(int dtype, size_t q, size_t p, const void* a, const size_t* n
         if (e != cudaSuccess) return cuda_fail(e, "kernel launch");
         if (!c_pinned && (e = cudaMemcpyAsync(c, hc.cbuf, need_c, cudaMemcpyDeviceToHost, hc.comp)) != cudaSuccess)
             return cuda_fail(e, "copy of C");
-        if ((e = cudaStreamSynchronize(hc.comp)) != cudaSuccess) return cuda_fail(e, "stream synchronize");
-        if (read_and_clear_device_error())
-            return fail(TLIBG_ERR_TIMEOUT, "tlibg: a bounded device wait expired; results are invalid");
-        return ok();
+        return finish();
     }
 
     // staged path: two chunk buffers in device memory (only this path needs them)
@@ -1375,10 +1479,7 @@ int tlibg_ttv_host(int dtype, size_t q, size_t p, const void* a, const size_t* n
     g_launches += launches;
     if (!c_pinned && (e = cudaMemcpyAsync(c, hc.cbuf, need_c, cudaMemcpyDeviceToHost, hc.comp)) != cudaSuccess)
         return cuda_fail(e, "copy of C");
-    if ((e = cudaStreamSynchronize(hc.comp)) != cudaSuccess) return cuda_fail(e, "stream synchronize");
-    unsigned int derr = read_and_clear_device_error();
-    if (derr) return fail(TLIBG_ERR_TIMEOUT, "tlibg: a bounded device wait expired; results are invalid");
-    return ok();
+    return finish();
 }
 
 // ---------------------------------------------------------------------------

@@ -26,6 +26,7 @@
 // rounding; this one reads A once whatever order is asked for.
 #include "ttv_internal.h"
 
+#include <algorithm>
 #include <string>
 #include <vector>
 
@@ -152,9 +153,9 @@ extern "C" int tlibg_ttvs(int dtype, size_t q, size_t p, const void* a, const si
             return internal_fail(TLIBG_ERR_UNSUPPORTED, "tlibg: a, b and c must be aligned to their element sizes");
     const int sms = internal_sms();
     if (!sms) return internal_fail(TLIBG_ERR_CUDA, "tlibg: no usable CUDA device");
-    if (int st = internal_check_device_pointers(a, c, c)) return st;
-    for (size_t r = 0; r + 1 < p; ++r)
-        if (int st = internal_check_device_pointers(bs[r], bs[r], bs[r])) return st;
+    if (int st = internal_check_device_pointers(a, c, bs[0])) return st;
+    for (size_t r = 1; r + 1 < p; r += 3)   // three pointers a check
+        if (int st = internal_check_device_pointers(bs[r], bs[std::min(r + 1, p - 2)], bs[std::min(r + 2, p - 2)])) return st;
 
     // modes in layout order, fastest first: extent and vector (q: none)
     std::vector<uint64_t> ext;
@@ -348,4 +349,19 @@ extern "C" int tlibg_ttvs(int dtype, size_t q, size_t p, const void* a, const si
     }
     internal_count_launches(launches);
     return internal_ok();
+}
+
+extern "C" int tlibg_ttvs_packed_rowmajor(const uint64_t* w)
+{
+    const size_t p = w[TLIBG_PACKED_P];
+    if (p < 2 || p > (size_t)KRON_MAX_MODES + 1)
+        return internal_fail(TLIBG_ERR_ARGUMENT, "tlibg_ttvs_packed_rowmajor: needs an order of 2 to 33");
+    const size_t* na = reinterpret_cast<const size_t*>(w + TLIBG_PACKED_WORDS);
+    const size_t *wa = na + p, *nbs = wa + p;
+    const void* const* bs = reinterpret_cast<const void* const*>(nbs + (p - 1));
+    size_t pia[KRON_MAX_MODES + 1];
+    for (size_t r = 0; r < p; ++r) pia[r] = p - r;
+    return tlibg_ttvs((int)w[TLIBG_PACKED_DTYPE], w[TLIBG_PACKED_Q], p, reinterpret_cast<const void*>(w[TLIBG_PACKED_A]), na,
+                      wa, pia, bs, nbs, reinterpret_cast<void*>(w[TLIBG_PACKED_C]),
+                      reinterpret_cast<void*>(w[TLIBG_PACKED_STREAM]));
 }

@@ -1143,6 +1143,11 @@ cudaError_t launch_wait_probe(cudaStream_t stream, uint32_t limit)
     return cudaGetLastError();
 }
 
+cudaError_t copy_device_error(unsigned int* dst, cudaStream_t stream)
+{
+    return cudaMemcpyFromSymbolAsync(dst, g_device_error, sizeof(unsigned int), 0, cudaMemcpyDeviceToHost, stream);
+}
+
 unsigned int read_and_clear_device_error()
 {
     unsigned int v = 0, zero = 0;

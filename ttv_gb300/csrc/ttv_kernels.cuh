@@ -176,6 +176,8 @@ size_t plan_smem_bytes(const Plan& p);
 int plan_ctas_per_sm(const Plan& p);
 
 unsigned int read_and_clear_device_error();
+// The error word into page-locked memory, in stream order (not cleared).
+cudaError_t copy_device_error(unsigned int* dst, cudaStream_t stream);
 
 // Self-test kernel: one bounded mbarrier wait that nothing completes.
 cudaError_t launch_wait_probe(cudaStream_t stream, uint32_t limit);
