@@ -841,3 +841,34 @@ def test_bounded_wait_expiry_reports_timeout(engine, orc, torch_dev):
     a = rng.uniform(-1, 1, int(np.prod(na))).astype(np.float32)
     b = rng.uniform(-1, 1, na[q - 1]).astype(np.float32)
     check(orc, engine, torch, dev, q, na, pia, a, b)
+
+
+@pytest.mark.parametrize("shape", [(512, 2048), (4096, 4095), (999, 1001), (256, 256, 64), (101, 300, 40), (2050, 700),
+                                   (64, 4, 160), (8, 40, 700), (2, 9, 14000), (4, 512, 8), (128, 128, 20), (513, 4, 3),
+                                   (16, 4, 1 << 20), (4100, 4, 4100)],
+                         ids=lambda s: "x".join(map(str, s)))
+def test_plans_on_the_general_stride_kernels(engine, orc, cuda, shape):
+    """fp32 calls around the lines where plans move to the general-stride kernels: rows, columns
+    (16-byte and single loads), thin prefixes and short contractions, first- and last-order, A on
+    and off the 16-byte grid.  Bar: Kahan's roundings, the merges' and the result's (4 x 2^-24 of
+    sum |a b|)."""
+    import torch
+    g = torch.Generator(device=cuda)
+    g.manual_seed(int(np.prod(shape)) % 100003)
+    p, N = len(shape), int(np.prod(shape))
+    buf = torch.rand(N + 1, generator=g, device=cuda) * 2 - 1
+    for pia in (list(range(1, p + 1)), list(range(p, 0, -1))):
+        wa = engine.strides(list(shape), pia)
+        for q in range(1, p + 1):
+            b = torch.rand(shape[q - 1], generator=g, device=cuda) * 2 - 1
+            nc, pic = engine.output_shape(list(shape), q), engine.output_layout(pia, q)
+            wc = engine.strides(nc, pic)
+            P, nq, S = orc.canonical(list(shape), pia, q)
+            for off in (0, 1):
+                if N > (1 << 24) and (off or pia[0] != 1):
+                    continue
+                a = buf[off:off + N]
+                c = torch.full((N // nq,), float("nan"), device=cuda)
+                engine.ttv(q, p, a, list(shape), wa, pia, b, [nq], c, nc, wc, pic, sync=True)
+                ref, absn = orc.truth(S, nq, P, a.cpu().numpy(), b.cpu().numpy())
+                assert orc.rel_error(c.cpu().numpy(), ref, absn) <= 4 * 2.0 ** -24, (pia, q, off)

@@ -5,7 +5,7 @@
 #include "ttv_internal.h"
 #include "ttv_kernels.cuh"
 #include "ttv_device.cuh"
-#include "ttv_general.cuh"
+#include "ttv_general.h"
 
 #include <algorithm>
 #include <atomic>
@@ -371,8 +371,62 @@ bool default_choices(const tlibg_options* opt)
 int make_plan_inner(int dtype, const Canon& cn, const void* a, const void* b, const tlibg_options* opt,
                     int sms, Plan* out);
 
+// fp32 plans that run faster on the general-stride kernels, which share the
+// contracted mode over warps and clusters without a second kernel and schedule
+// many short columns as many CTAs.  Measured against the dense plan on 4 to 256 MB
+// (device time, inputs rotated through L2):
+//   rows split by the plan, A up to 2^26 elements: 1.3 to 2.5 times as fast below
+//     2^24 (512 x 4096: 6.9 -> 2.9 us, 4096 x 4096: 15.9 -> 11.4), level at 2^26;
+//   columns split by the plan: 16-byte loads up to 2^25 elements (256^3: 17.5 ->
+//     13.4 us, 2^25: 30 -> 25; 19404 x 1777 above it 29 -> 38), narrower ones up
+//     to 2^23 (2050 x 2730 x 3 from there on the dense kernel wins);
+//   thin prefixes with slabs of at most 2^14 elements, more of them than SMs or
+//     split by the plan (64 x 4 x 4096: 9.9 -> 2.3 us, 128^3: 5.5 -> 4.1; longer
+//     slabs are 1.4 to 4 times slower here), prefixes under 8 elements only where
+//     A is small;
+//   contractions of at most 4 rows, A of 2^26 elements or more and a prefix of 16
+//     (2^28: 208 -> 197 us, 2^25: level, 2^23: 7.0 -> 8.4; a prefix of 4: 84 -> 112).
+// Contractions over more than 2^20 elements keep the fp64 combine.
+void route_general(const Canon& cn, const void* a, const void* b, int sms, Plan* pl)
+{
+    if (pl->dtype != F32 || !pl->kahan || cn.nq > (uint64_t(1) << 20)) return;
+    const uint64_t elems = cn.P * cn.nq * cn.S;
+    bool take = false;
+    if (pl->kind == KIND_ROW) {
+        take = pl->split > 1 && elems <= (uint64_t(1) << 26);
+    } else if (pl->kind == KIND_COL_THIN) {
+        take = (cn.S > (uint64_t)sms || pl->split > 1) && cn.nq * cn.P <= (uint64_t(1) << 14) &&
+               (cn.P >= 8 || elems <= (uint64_t(1) << 18));
+    } else if (pl->kind == KIND_COL) {
+        if (pl->rows_m == 1) take = elems >= (uint64_t(1) << 26) && cn.P >= 16;
+        else take = pl->split > 1 && elems <= (uint64_t(1) << (pl->vec == 4 ? 25 : 23));
+    }
+    if (!take) return;
+    GSPlan g;
+    std::vector<std::tuple<size_t, size_t, size_t>> modes;
+    if (cn.P > 1) modes.emplace_back(1, cn.P, 1);
+    if (cn.S > 1) modes.emplace_back(cn.nq * cn.P, cn.S, cn.P);
+    gs_modes(std::move(modes), &g.k);
+    g.k.a = a;
+    g.k.b = b;
+    g.k.nq = cn.nq;
+    g.k.waq = cn.nq > 1 ? cn.P : 0;
+    g.k.wb = 1;
+    gs_plan(sms, &g);
+    pl->general = true;
+    pl->kind = g.row ? KIND_ROW : KIND_COL;
+    pl->rows_m = 0;
+    pl->group = g.row ? 1 << g.k.group_log2 : 1 << g.k.wi_log2;
+    pl->vec = g.V;
+    pl->split = (int)g.k.nseg;
+    pl->grid = g.grid;
+    pl->f64_combine = false;
+    pl->smem = 0;
+    pl->gs = g;
+}
+
 int make_plan(int dtype, const Canon& cn, const void* a, const void* b, const tlibg_options* opt,
-              int sms, Plan* out)
+              int sms, Plan* out, bool general = true)
 {
     if (default_choices(opt)) {
         tlibg_options hinted;
@@ -395,7 +449,9 @@ int make_plan(int dtype, const Canon& cn, const void* a, const void* b, const tl
             }
         }
     }
-    return make_plan_inner(dtype, cn, a, b, opt, sms, out);
+    const int st = make_plan_inner(dtype, cn, a, b, opt, sms, out);
+    if (st == TLIBG_OK && general && default_choices(opt)) route_general(cn, a, b, sms, out);
+    return st;
 }
 
 // TMA-staged column kernel: items (segment, slice, tile of 4 KB of a row), a
@@ -751,6 +807,10 @@ int make_plan_inner(int dtype, const Canon& cn, const void* a, const void* b, co
             Plan probe = pl;
             probe.group = 1;
             thin = cdiv(outputs, TO1) < (uint64_t)sms * std::max(1, plan_ctas_per_sm(probe));
+            // a slab of less than one step of the CTA's warps leaves most of them idle; a CTA
+            // per slab is still the shortest launch while each SM gets one at most (fp64 832
+            // slabs of 4 x 4: 8.7 -> 3.4 us; 24 of 20 x 16 fp32 2.3, without it 2.7)
+            thin = thin && (cn.S <= (uint64_t)sms || cn.nq >= (BLOCK / 32) * (32 / PV));
         }
         if (thin) {
             pl.kind = KIND_COL_THIN;
@@ -1213,7 +1273,7 @@ int tlibg_ttv_strided(int dtype, size_t q, size_t p, const void* a, const size_t
     pl.f64 = dtype == F64;
     gs_plan(sms, &pl);
     if (pl.k.nseg > 1)
-        if (int s = get_scratch(st, (size_t)pl.k.nseg * pl.k.outputs * 2 * elem_size_t(dtype), &pl.k.part)) return s;
+        if (int s = get_scratch(st, gs_partial_bytes(pl), &pl.k.part)) return s;
     uint64_t launches = 0;
     const cudaError_t e = gs_launch(pl, st, sms, &launches);
     g_launches += launches;
@@ -1382,7 +1442,7 @@ int tlibg_ttv_host(int dtype, size_t q, size_t p, const void* a, const size_t* n
         if (opt) o2 = *opt;
         if (o2.kind == KIND_STREAM || o2.kind == KIND_ROW_TILE || o2.kind == KIND_COL_BULK) o2.kind = -1;
         Plan probe_pl;
-        if ((st = make_plan(dtype, cn, at.devicePointer, hc.bbuf, &o2, d.sms, &probe_pl))) return st;
+        if ((st = make_plan(dtype, cn, at.devicePointer, hc.bbuf, &o2, d.sms, &probe_pl, false))) return st;
         // a warp's 16-byte loads cover one 512-byte run: column tiles, thin prefixes of
         // at least 512 bytes, rows taken by a whole warp
         const bool v16 = (size_t)probe_pl.vec * ea == 16;
@@ -1401,10 +1461,10 @@ int tlibg_ttv_host(int dtype, size_t q, size_t p, const void* a, const size_t* n
         if (opt) o2 = *opt;
         if (o2.kind == KIND_STREAM || o2.kind == KIND_ROW_TILE || o2.kind == KIND_COL_BULK) o2.kind = -1;
         Plan pl;
-        if ((st = make_plan(dtype, cn, at.devicePointer, hc.bbuf, &o2, d.sms, &pl))) return st;
+        if ((st = make_plan(dtype, cn, at.devicePointer, hc.bbuf, &o2, d.sms, &pl, false))) return st;
         if (pl.kind == KIND_STREAM || pl.kind == KIND_ROW_TILE || pl.kind == KIND_COL_BULK) {
             o2.kind = cn.P == 1 ? KIND_ROW : KIND_COL;
-            if ((st = make_plan(dtype, cn, at.devicePointer, hc.bbuf, &o2, d.sms, &pl))) return st;
+            if ((st = make_plan(dtype, cn, at.devicePointer, hc.bbuf, &o2, d.sms, &pl, false))) return st;
         }
         void* part = nullptr;
         if ((st = get_scratch(hc.comp, partial_bytes(pl), &part))) return st;
@@ -1467,7 +1527,7 @@ int tlibg_ttv_host(int dtype, size_t q, size_t p, const void* a, const size_t* n
         Canon ck = cn;
         ck.S = sn;
         Plan pl;
-        if ((st = make_plan(dtype, ck, adev, hc.bbuf, opt, d.sms, &pl))) return st;
+        if ((st = make_plan(dtype, ck, adev, hc.bbuf, opt, d.sms, &pl, false))) return st;
         void* part = nullptr;
         if ((st = get_scratch(hc.comp, partial_bytes(pl), &part))) return st;
         // page-locked C: each chunk's kernels store their part of C in place

@@ -1,4 +1,4 @@
-// General-stride TTV (included by ttv_api.cu): tlibg_ttv_strided, an extension
+// General-stride TTV kernels: tlibg_ttv_strided, an extension
 // beside the drop-in calls with the natural meaning of every stride -- A's
 // element (i_1..i_p) at a[sum_r i_r wa[r]], b's element i at b[i wb], C's
 // element (j_1..j_{p-1}) at c[sum_r j_r wc[r]] -- for views (sliced, padded,
@@ -28,7 +28,8 @@
 // 128-bit fixed point (FxAcc), because GB300 issues two FP64 instructions per
 // SM and clock: Kahan's four per element cap a view at 1.2 TB/s, the one
 // multiply left here at 4.7.
-#pragma once
+#include "ttv_general.h"
+#include "ttv_device.cuh"
 
 #include <cooperative_groups.h>
 
@@ -41,9 +42,6 @@
 
 namespace tlibg {
 
-constexpr int GS_MAX_MODES = 16;   // modes other than q
-constexpr int GS_MAX_CLUSTER = 8;
-
 // Resident CTAs per SM the kernels are compiled for.  An unshared fp32 kernel
 // lives off warps in flight: 6 for one-element columns (38 x 814,000 outputs:
 // 30.9 us, 42 when the shared form's code held it to 4), 4 for 16-byte columns
@@ -55,26 +53,6 @@ template <typename T, int N, bool SHARE> constexpr int gs_col_ctas()
     return sizeof(T) == 4 && !SHARE && N == 1 ? 6 : 4;
 }
 template <typename T> constexpr int gs_row_ctas() { return sizeof(T) == 8 ? 3 : 4; }
-
-struct GSArgs {
-    const void* a;
-    const void* b;
-    void* c;
-    void* part;                   // pairs [nseg][outputs] when nseg > 1
-    uint64_t wa[GS_MAX_MODES];    // strides of the modes other than q, A-stride order
-    uint64_t wc[GS_MAX_MODES];
-    IdxDiv ext[GS_MAX_MODES];     // their extents, as divisors
-    int nm;
-    uint64_t outputs;             // product of the extents
-    uint64_t nq, waq, wb;
-    uint64_t tiles, items;        // tiles of outputs; items = tiles x nseg
-    uint64_t seg_len, sub_len;    // rows of q per segment, and per CTA of a cluster
-    IdxDiv tdiv;                  // items -> segment
-    uint32_t nseg;
-    uint32_t cluster_log2;        // CTAs of a cluster, all along q
-    uint32_t wi_log2;             // warps along q
-    uint32_t group_log2;          // row form: lanes per output
-};
 
 // Offsets of output o in A and in C.  All the extents' divisors are of one kind
 // (one dividend bound), so 32-bit index arithmetic serves all modes or none.
@@ -668,17 +646,9 @@ template <typename T> __global__ void __launch_bounds__(256) gs_combine_kernel(G
 // --------------------------------------------------------------------------
 // host side: plan and launch
 // --------------------------------------------------------------------------
-struct GSPlan {
-    GSArgs k{};
-    bool f64 = false, row = false;
-    bool fx = false;        // fp64: fixed-point sums (else Kahan)
-    int V = 1, M = 1;       // vector width; vectors per thread (column) or rows per group (row)
-    int grid = 1;
-};
-
 // Modes other than q as (A stride, extent, C stride), sorted; extents of 1 left
 // out.  Neighbours merge when one stride steps through both in A and in C.
-inline void gs_modes(std::vector<std::tuple<size_t, size_t, size_t>> modes, GSArgs* k)
+void gs_modes(std::vector<std::tuple<size_t, size_t, size_t>> modes, GSArgs* k)
 {
     std::sort(modes.begin(), modes.end());
     k->nm = 0;
@@ -702,7 +672,7 @@ inline void gs_modes(std::vector<std::tuple<size_t, size_t, size_t>> modes, GSAr
 // The plan's kernel, and the loads each of its lanes keeps in flight per row or
 // vector of outputs (U).
 typedef void (*GsFn)(GSArgs);
-template <bool SHARE> inline GsFn gs_kernel_of(const GSPlan& p, int& U)
+template <bool SHARE> static GsFn gs_kernel_of(const GSPlan& p, int& U)
 {
     const int M = p.M;
     if (p.f64) {
@@ -732,7 +702,7 @@ template <bool SHARE> inline GsFn gs_kernel_of(const GSPlan& p, int& U)
     return M == 4 ? gs_col_kernel<float, 1, 4, 4, false, SHARE>
                   : (M == 2 ? gs_col_kernel<float, 1, 2, 8, false, SHARE> : gs_col_kernel<float, 1, 1, 8, false, SHARE>);
 }
-inline GsFn gs_kernel(const GSPlan& p, bool share, int* u = nullptr)
+static GsFn gs_kernel(const GSPlan& p, bool share, int* u = nullptr)
 {
     int U = 1;
     const GsFn fn = share ? gs_kernel_of<true>(p, U) : gs_kernel_of<false>(p, U);
@@ -741,7 +711,7 @@ inline GsFn gs_kernel(const GSPlan& p, bool share, int* u = nullptr)
 }
 
 // Resident CTAs per SM of a plan's kernel (3 without a device), cached.
-inline int gs_ctas_per_sm(const GSPlan& p, bool share)
+static int gs_ctas_per_sm(const GSPlan& p, bool share)
 {
     const void* fn = reinterpret_cast<const void*>(gs_kernel(p, share));
     static std::mutex mu;
@@ -767,7 +737,7 @@ inline int gs_ctas_per_sm(const GSPlan& p, bool share)
 // (clocks swept from 1200 to 2000, the cost of sharing from 600 to 5500).
 // `rows`: loads along q of an unsplit warp (row form: of a lane); N: elements a
 // lane loads per row.
-inline void gs_split(GSPlan* p, uint64_t rows, bool may_split, uint32_t outs_per_warp, int N, int sms)
+static void gs_split(GSPlan* p, uint64_t rows, bool may_split, uint32_t outs_per_warp, int N, int sms)
 {
     GSArgs& k = p->k;
     int U = 1;
@@ -817,7 +787,7 @@ inline void gs_split(GSPlan* p, uint64_t rows, bool may_split, uint32_t outs_per
     p->grid = (int)(std::min<uint64_t>(k.items, ((uint64_t)sms * 32) >> k.cluster_log2) << k.cluster_log2);
 }
 
-inline void gs_plan(int sms, GSPlan* p)
+void gs_plan(int sms, GSPlan* p)
 {
     GSArgs& k = p->k;
     const uint64_t V = p->f64 ? 2 : 4;
@@ -864,20 +834,23 @@ inline void gs_plan(int sms, GSPlan* p)
     }
 }
 
-inline cudaError_t gs_launch(const GSPlan& p, cudaStream_t st, int sms, uint64_t* launches)
+cudaError_t gs_launch(const GSPlan& p, cudaStream_t st, int sms, uint64_t* launches, bool dependent)
 {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)p.grid);
     cfg.blockDim = dim3(256);
     cfg.stream = st;
-    cudaLaunchAttribute attr[1];
+    cudaLaunchAttribute attr[2];
     cfg.attrs = attr;
+    if (dependent) {
+        attr[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[cfg.numAttrs++].val.programmaticStreamSerializationAllowed = 1;
+    }
     if (p.k.cluster_log2 > 0) {
-        attr[0].id = cudaLaunchAttributeClusterDimension;
-        attr[0].val.clusterDim.x = 1u << p.k.cluster_log2;
-        attr[0].val.clusterDim.y = 1;
-        attr[0].val.clusterDim.z = 1;
-        cfg.numAttrs = 1;
+        attr[cfg.numAttrs].id = cudaLaunchAttributeClusterDimension;
+        attr[cfg.numAttrs].val.clusterDim.x = 1u << p.k.cluster_log2;
+        attr[cfg.numAttrs].val.clusterDim.y = 1;
+        attr[cfg.numAttrs++].val.clusterDim.z = 1;
     }
     cudaError_t e = cudaLaunchKernelEx(&cfg, gs_kernel(p, p.k.wi_log2 > 0), p.k);
     if (e != cudaSuccess) return e;

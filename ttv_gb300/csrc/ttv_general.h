@@ -1,0 +1,61 @@
+// Plan and launch interface of the general-stride kernels (ttv_general.cu).
+#pragma once
+
+#include "ttv_idxdiv.h"
+
+#include <cuda_runtime.h>
+#include <stdint.h>
+
+#include <tuple>
+#include <vector>
+
+namespace tlibg {
+
+constexpr int GS_MAX_MODES = 16;   // modes other than q
+constexpr int GS_MAX_CLUSTER = 8;
+
+struct GSArgs {
+    const void* a;
+    const void* b;
+    void* c;
+    void* part;                   // pairs [nseg][outputs] when nseg > 1
+    uint64_t wa[GS_MAX_MODES];    // strides of the modes other than q, A-stride order
+    uint64_t wc[GS_MAX_MODES];
+    IdxDiv ext[GS_MAX_MODES];     // their extents, as divisors
+    int nm;
+    uint64_t outputs;             // product of the extents
+    uint64_t nq, waq, wb;
+    uint64_t tiles, items;        // tiles of outputs; items = tiles x nseg
+    uint64_t seg_len, sub_len;    // rows of q per segment, and per CTA of a cluster
+    IdxDiv tdiv;                  // items -> segment
+    uint32_t nseg;
+    uint32_t cluster_log2;        // CTAs of a cluster, all along q
+    uint32_t wi_log2;             // warps along q
+    uint32_t group_log2;          // row form: lanes per output
+};
+
+struct GSPlan {
+    GSArgs k{};
+    bool f64 = false, row = false;
+    bool fx = false;        // fp64: fixed-point sums (else Kahan)
+    int V = 1, M = 1;       // vector width; vectors per thread (column) or rows per group (row)
+    int grid = 1;
+};
+
+// The modes other than q as (A stride, extent, C stride); extents of 1 left out.
+void gs_modes(std::vector<std::tuple<size_t, size_t, size_t>> modes, GSArgs* k);
+
+// Form, vector width and split for the args' modes, a, b, nq, waq and wb.
+void gs_plan(int sms, GSPlan* p);
+
+// Enqueues a plan's kernels; `dependent`: as a programmatic dependent of the
+// stream's previous kernel.
+cudaError_t gs_launch(const GSPlan& p, cudaStream_t st, int sms, uint64_t* launches, bool dependent = false);
+
+// Bytes of partial sums the plan needs (args.part), 0 without segments.
+inline size_t gs_partial_bytes(const GSPlan& p)
+{
+    return p.k.nseg > 1 ? (size_t)p.k.nseg * p.k.outputs * 2 * (p.f64 ? 8 : 4) : 0;
+}
+
+}  // namespace tlibg

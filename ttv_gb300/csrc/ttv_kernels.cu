@@ -938,6 +938,7 @@ size_t plan_smem_bytes(const Plan& p)
 
 size_t partial_bytes(const Plan& p)
 {
+    if (p.general) return gs_partial_bytes(p.gs);
     if (p.split <= 1) return 0;
     return (size_t)p.split * p.S * p.P * 2 * acc_size(p.dtype);
 }
@@ -1002,6 +1003,17 @@ static cudaError_t launch_ex(void (*fn)(Params...), int grid, int threads, size_
 cudaError_t launch_plan(const Plan& plan, const void* a, const void* b, void* c, void* partial,
                         cudaStream_t stream, uint64_t* launches, bool dependent)
 {
+    if (plan.general) {
+        GSPlan g = plan.gs;
+        g.k.a = a;
+        g.k.b = b;
+        g.k.c = c;
+        g.k.part = partial;
+        uint64_t n = 0;
+        const cudaError_t err = gs_launch(g, stream, plan.sms, &n, dependent);
+        if (launches) *launches += n;
+        return err;
+    }
     if (plan.kind == KIND_STREAM) {
         SArgs sa;
         sa.a = a;

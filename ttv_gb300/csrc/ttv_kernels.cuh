@@ -4,6 +4,9 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "ttv_general.h"
+#include "ttv_idxdiv.h"
+
 namespace tlibg {
 
 enum DType { F32 = 0, F64 = 1, BF16A = 2 };
@@ -79,6 +82,9 @@ struct Plan {
     int stream_col = 0;          // 0: row form (P == 1), 1: column form
     uint64_t L = 0, R = 0, units = 0, units_per_cta = 0;
     int RG = 1, J = 1;
+    // ROW / COL: runs on the general-stride kernels (ttv_general.cu), `gs` its plan
+    bool general = false;
+    GSPlan gs;
 };
 
 // Row-shift kernel (rows that are not whole 16-byte vectors): V shifted copies
@@ -95,51 +101,6 @@ __host__ __device__ inline size_t rs_smem_bytes(uint64_t nq, size_t es, bool spl
 
 // Whether the streamed kernel can take a problem (whole rows fit a stage).
 bool stream_eligible(int dtype, uint64_t P, uint64_t nq);
-
-// --------------------------------------------------------------------------
-// division by a divisor fixed for a launch (output -> slice, item -> segment)
-// --------------------------------------------------------------------------
-// When every dividend and the divisor fit 32 bits, n / d is one multiply-high,
-// a subtract, an add and two shifts: the round-up method of Granlund and
-// Montgomery ("Division by invariant integers using multiplication", PLDI
-// 1994, section 4) with l = ceil(log2 d), m = floor(2^32 (2^l - d) / d) + 1,
-// t = hi32(m n), n / d = (t + ((n - t) >> min(l, 1))) >> max(l - 1, 0).
-// Otherwise the plain 64-bit division.  Built on the host per launch (and on
-// the device per problem by the batched executor's planning kernel).
-struct IdxDiv {
-    uint64_t d;
-    uint32_t m;
-    uint8_t s1, s2, fast;
-};
-
-__host__ __device__ inline IdxDiv make_idx_div(uint64_t d, uint64_t max_dividend)
-{
-    IdxDiv v{d == 0 ? 1 : d, 0, 0, 0, 0};
-    if (v.d < (uint64_t(1) << 32) && max_dividend < (uint64_t(1) << 32)) {
-        uint32_t l = 0;
-        while ((uint64_t(1) << l) < v.d) ++l;
-        v.m = (uint32_t)(((uint64_t(1) << 32) * ((uint64_t(1) << l) - v.d)) / v.d + 1);
-        v.s1 = (uint8_t)(l < 1 ? l : 1);
-        v.s2 = (uint8_t)(l > 0 ? l - 1 : 0);
-        v.fast = 1;
-    }
-    return v;
-}
-
-// (Host-callable too, so the CPU tests run this very code.)
-__host__ __device__ __forceinline__ uint64_t idx_div(uint64_t n, const IdxDiv& v)
-{
-    if (v.fast) {
-        const uint32_t x = (uint32_t)n;
-#ifdef __CUDA_ARCH__
-        const uint32_t t = __umulhi(v.m, x);
-#else
-        const uint32_t t = (uint32_t)(((uint64_t)v.m * x) >> 32);
-#endif
-        return (t + ((x - t) >> v.s1)) >> v.s2;
-    }
-    return n / v.d;
-}
 
 struct KArgs {
     const void* a;
