@@ -872,3 +872,31 @@ def test_plans_on_the_general_stride_kernels(engine, orc, cuda, shape):
                 engine.ttv(q, p, a, list(shape), wa, pia, b, [nq], c, nc, wc, pic, sync=True)
                 ref, absn = orc.truth(S, nq, P, a.cpu().numpy(), b.cpu().numpy())
                 assert orc.rel_error(c.cpu().numpy(), ref, absn) <= 4 * 2.0 ** -24, (pia, q, off)
+
+
+@pytest.mark.parametrize("dtype", ["f32", "f64", "bf16"])
+@pytest.mark.parametrize("P", [1, 2, 3, 5, 6, 7, 12, 24, 33, 40, 56, 100, 120])
+def test_thin_prefixes_of_any_width(engine, orc, cuda, P, dtype):
+    """Thin prefixes whose vectors divide the warp and not (idle lanes), one to several slabs,
+    contractions of one row to several segments, around the lines to the column kernels.  Bars:
+    fp32 and bf16 storage 4 x 2^-24 of sum |a b|; fp64 the suite's 1e-13."""
+    import torch
+    g = torch.Generator(device=cuda)
+    g.manual_seed(P)
+    dt = {"f32": engine.F32, "f64": engine.F64, "bf16": engine.BF16A}[dtype]
+    tdt = torch.float64 if dtype == "f64" else torch.float32
+    for nq, S in ((1, 1), (2, 3), (31, 2), (4097, 1), (90001, 1), (20000, 4), (700, 20), (9, 700), (130, 620)):
+        N = P * nq * S
+        a = torch.rand(N, generator=g, device=cuda, dtype=tdt) * 2 - 1
+        if dtype == "bf16":
+            a = a.to(torch.bfloat16)
+        b = torch.rand(nq, generator=g, device=cuda, dtype=tdt) * 2 - 1
+        c = torch.full((P * S,), float("nan"), device=cuda, dtype=tdt)
+        na, pia = [P, nq, S], [1, 2, 3]
+        wa = engine.strides(na, pia)
+        nc, pic = engine.output_shape(na, 2), engine.output_layout(pia, 2)
+        engine.ttv(2, 3, a.view(torch.int16) if dtype == "bf16" else a, na, wa, pia, b, [nq], c, nc,
+                   engine.strides(nc, pic), pic, dtype=dt, sync=True)
+        ref, absn = orc.truth(S, nq, P, a.double().cpu().numpy(), b.double().cpu().numpy())
+        bar = 1e-13 if dtype == "f64" else 4 * 2.0 ** -24
+        assert orc.rel_error(c.cpu().numpy(), ref, absn) <= bar, (nq, S)

@@ -378,12 +378,13 @@ int make_plan_inner(int dtype, const Canon& cn, const void* a, const void* b, co
 //   rows split by the plan, A up to 2^26 elements: 1.3 to 2.5 times as fast below
 //     2^24 (512 x 4096: 6.9 -> 2.9 us, 4096 x 4096: 15.9 -> 11.4), level at 2^26;
 //   columns split by the plan: 16-byte loads up to 2^25 elements (256^3: 17.5 ->
-//     13.4 us, 2^25: 30 -> 25; 19404 x 1777 above it 29 -> 38), narrower ones up
-//     to 2^23 (2050 x 2730 x 3 from there on the dense kernel wins);
+//     13.4 us, 2^25: 30 -> 25; 19404 x 1777 above it 29 -> 38), prefixes under 48
+//     up to 2^21 (40 x 5242 x 20: 9.2 -> 10.8), narrower loads up to 2^23 (from
+//     2050 x 2730 x 3 on the dense kernel wins);
 //   thin prefixes with slabs of at most 2^14 elements, more of them than SMs or
 //     split by the plan (64 x 4 x 4096: 9.9 -> 2.3 us, 128^3: 5.5 -> 4.1; longer
-//     slabs are 1.4 to 4 times slower here), prefixes under 8 elements only where
-//     A is small;
+//     slabs are 1.4 to 4 times slower here), prefixes under 8 elements only many
+//     slabs of a small A (2 x 2138 x 16: 4.2 -> 5.7);
 //   contractions of at most 4 rows, A of 2^26 elements or more and a prefix of 16
 //     (2^28: 208 -> 197 us, 2^25: level, 2^23: 7.0 -> 8.4; a prefix of 4: 84 -> 112).
 // Contractions over more than 2^20 elements keep the fp64 combine.
@@ -395,11 +396,11 @@ void route_general(const Canon& cn, const void* a, const void* b, int sms, Plan*
     if (pl->kind == KIND_ROW) {
         take = pl->split > 1 && elems <= (uint64_t(1) << 26);
     } else if (pl->kind == KIND_COL_THIN) {
-        take = (cn.S > (uint64_t)sms || pl->split > 1) && cn.nq * cn.P <= (uint64_t(1) << 14) &&
-               (cn.P >= 8 || elems <= (uint64_t(1) << 18));
+        take = cn.nq * cn.P <= (uint64_t(1) << 14) &&
+               (cn.P >= 8 ? cn.S > (uint64_t)sms || pl->split > 1 : cn.S > (uint64_t)sms && elems <= (uint64_t(1) << 18));
     } else if (pl->kind == KIND_COL) {
         if (pl->rows_m == 1) take = elems >= (uint64_t(1) << 26) && cn.P >= 16;
-        else take = pl->split > 1 && elems <= (uint64_t(1) << (pl->vec == 4 ? 25 : 23));
+        else take = pl->split > 1 && elems <= (uint64_t(1) << (pl->vec < 4 ? 23 : (cn.P >= 48 ? 25 : 21)));
     }
     if (!take) return;
     GSPlan g;
@@ -801,7 +802,14 @@ int make_plan_inner(int dtype, const Canon& cn, const void* a, const void* b, co
             return fail(TLIBG_ERR_ARGUMENT, "tlibg: the thin-prefix column kernel needs P / vector width "
                                             "to divide 32");
         bool thin = opt && opt->kind == KIND_COL_THIN;
-        if (!thin && thin_shape && !(opt && opt->kind >= 0)) {
+        // Prefixes whose vectors do not divide the warp (its last lanes idle): where the slabs
+        // are few, so that the column kernel's split would leave each warp a prefix's few lanes
+        // (measured at 1 to 1000 slabs of 2^14 to 2^25 elements: up to 4 slabs 1.2 to 9 times
+        // as fast, 20 slabs of 3 to 7 1.2 to 1.7 in fp32 and bf16, beyond that 0.5 to 0.9)
+        const bool thin_ragged = pl.kind == KIND_COL && cn.P % V == 0 && PV <= 16 && 32 % PV != 0 &&
+                                 (dtype != F32 || cn.P <= 32) &&
+                                 (cn.S <= 4 || cn.S * cn.P <= (dtype == F64 ? 64u : 160u));
+        if (!thin && (thin_shape || thin_ragged) && !(opt && opt->kind >= 0)) {
             // few outputs: the plain column kernel would leave most lanes idle
             const uint64_t TO1 = (uint64_t)(BLOCK / 32) * 32 * V;
             Plan probe = pl;
@@ -811,6 +819,16 @@ int make_plan_inner(int dtype, const Canon& cn, const void* a, const void* b, co
             // per slab is still the shortest launch while each SM gets one at most (fp64 832
             // slabs of 4 x 4: 8.7 -> 3.4 us; 24 of 20 x 16 fp32 2.3, without it 2.7)
             thin = thin && (cn.S <= (uint64_t)sms || cn.nq >= (BLOCK / 32) * (32 / PV));
+            // Many slabs: a CTA reduces through shared memory once per slab, which small slabs
+            // do not pay for.  Column kernel from 4 slabs per SM on (fp64: also from one, where
+            // a slab is long enough for its split): fp64 1000 slabs of 4 x 512 13.6 -> 8.7 us,
+            // 4000 of 16 x 128 33.7 -> 21.3, 200 of 16 x 2048 22.8 -> 18.0; bf16 4000 of
+            // 16 x 128 27.0 -> 10.0, of 16 x 512 32.7 -> 28.0 but of 4 x 2048 27.3 -> 52.0.
+            const uint64_t slab = cn.P * cn.nq;
+            if (dtype == F64)
+                thin = thin && !(cn.S > (uint64_t)sms && slab <= (1u << 15) && (cn.S >= 4 * (uint64_t)sms || slab >= (1u << 13)));
+            else if (dtype == BF16A)
+                thin = thin && !(cn.S >= 4 * (uint64_t)sms && slab <= (1u << 12));
         }
         if (thin) {
             pl.kind = KIND_COL_THIN;

@@ -1,10 +1,13 @@
 // Column kernel for thin prefixes (included by ttv_kernels.cu).
 //
-// When P is small (P / V lanes cover a row of the prefix and P / V divides
-// 32) and there are too few outputs S * P to give every lane of the plain
-// column kernel an output, a warp reads RG = 32 V / P consecutive rows of a
-// slab per step: lane L owns outputs j = (L mod P/V) * V .. + V - 1 of row
-// group g = L / (P/V), so each warp load covers 32 V contiguous elements.
+// When P is small (P / V <= 32 lanes cover a row of the prefix) and there are
+// too few outputs S * P to give every lane of the plain column kernel an
+// output, a warp reads RG = 32 / (P / V) consecutive rows of a slab per step:
+// lane L owns outputs j = (L mod P/V) * V .. + V - 1 of row group
+// g = L / (P/V), so each warp load covers RG P contiguous elements (where P / V
+// does not divide 32 the last lanes idle: 30 of 32 work on prefixes of 24 floats
+// or of 3, of which a column-kernel warp reads one row at a time: 24 x 466033 x 3
+// fp32 67.9 -> 28.8 us, bf16 105 -> 24.8, 3 x 1398101 fp64 219 -> 23.7).
 // The 8 warps of a CTA interleave along the contracted mode; a work item is
 // one (segment of q, slab s).  Lanes of the same outputs are reduced by
 // shuffles, the warps through shared memory in fixed order, segments by the
@@ -34,7 +37,8 @@ __global__ void __launch_bounds__(BLOCK, (min_ctas<TA, V>())) col_thin_kernel(KA
     const uint64_t P = k.P;
     const uint32_t PV = (uint32_t)(P / V);   // lanes per row
     const uint32_t RG = 32u / PV;            // rows per warp step
-    const uint32_t g = lane / PV;
+    const uint32_t g = lane / PV;            // row group; RG: an idle lane
+    const bool whole = PV * RG == 32u;       // every lane works
     const uint64_t j0 = (uint64_t)(lane % PV) * V;
     const uint32_t step = NW * RG;           // rows between a lane's consecutive loads
     const TA* __restrict__ A = static_cast<const TA*>(k.a);
@@ -72,23 +76,39 @@ __global__ void __launch_bounds__(BLOCK, (min_ctas<TA, V>())) col_thin_kernel(KA
 #pragma unroll
         for (int v = 0; v < V; ++v) acc[v].init();
         const TA* ap = A + s * k.nq * P + j0;
+        const uint64_t i0 = g < RG ? ib + warp * RG + g : ie;
         if constexpr (PRES) {
             if (b_split_ok)
-                col_loop<U, V, true>(acc, ap, P, bs, bsp, ib + warp * RG + g, ie, step);
+                col_loop<U, V, true>(acc, ap, P, bs, bsp, i0, ie, step);
             else
-                col_loop<U, V, false>(acc, ap, P, bs, bsp, ib + warp * RG + g, ie, step);
+                col_loop<U, V, false>(acc, ap, P, bs, bsp, i0, ie, step);
         } else {
-            col_loop<U, V, false>(acc, ap, P, bs, bsp, ib + warp * RG + g, ie, step);
+            col_loop<U, V, false>(acc, ap, P, bs, bsp, i0, ie, step);
         }
 #pragma unroll
         for (int v = 0; v < V; ++v) acc[v].fold();
         // lanes of the same outputs (row groups g) in the warp, then the warps
-        for (uint32_t o = PV; o < 32u; o <<= 1) {
+        if (whole) {
+            for (uint32_t o = PV; o < 32u; o <<= 1) {
 #pragma unroll
-            for (int v = 0; v < V; ++v) {
-                const T os = __shfl_xor_sync(0xffffffffu, acc[v].s, o);
-                const T oc = __shfl_xor_sync(0xffffffffu, acc[v].c, o);
-                acc[v].merge(os, oc);
+                for (int v = 0; v < V; ++v) {
+                    const T os = __shfl_xor_sync(0xffffffffu, acc[v].s, o);
+                    const T oc = __shfl_xor_sync(0xffffffffu, acc[v].c, o);
+                    acc[v].merge(os, oc);
+                }
+            }
+        } else {
+            // groups h .. n - 1 into groups 0 .., h the powers of two below n
+            uint32_t n = RG;
+            for (uint32_t h = 16; h > 0; h >>= 1) {
+                if (h >= n) continue;
+#pragma unroll
+                for (int v = 0; v < V; ++v) {
+                    const T os = __shfl_down_sync(0xffffffffu, acc[v].s, h * PV);
+                    const T oc = __shfl_down_sync(0xffffffffu, acc[v].c, h * PV);
+                    if (g < h && g + h < n) acc[v].merge(os, oc);
+                }
+                n = h;
             }
         }
         if (lane < PV) {
