@@ -874,6 +874,41 @@ def test_plans_on_the_general_stride_kernels(engine, orc, cuda, shape):
                 assert orc.rel_error(c.cpu().numpy(), ref, absn) <= 4 * 2.0 ** -24, (pia, q, off)
 
 
+@pytest.mark.parametrize("shape", [(512, 2048), (96, 700), (88, 700), (1001, 530), (32776, 17), (32776, 140), (256, 256, 32),
+                                   (101, 300, 40), (2050, 70), (4097, 4097), (64, 4, 160), (8, 40, 700), (6, 4, 300),
+                                   (1026, 3, 9), (513, 4, 3), (16, 4, 4)], ids=lambda s: "x".join(map(str, s)))
+def test_bf16_plans_on_the_general_stride_kernels(engine, orc, cuda, shape):
+    """bf16-stored A around the same lines: rows of 96, split rows, thin prefixes, columns in 16-byte,
+    4-byte and single loads, A on and off the 16- and the 4-byte grid; non-finite elements land in
+    their own outputs.  Bar: 4 x 2^-24 of sum |a b| (products and sums are fp32, Kahan)."""
+    import torch
+    g = torch.Generator(device=cuda)
+    g.manual_seed(int(np.prod(shape)) % 100003)
+    p, N = len(shape), int(np.prod(shape))
+    buf = (torch.rand(N + 2, generator=g, device=cuda) * 2 - 1).to(torch.bfloat16)
+    for pia in (list(range(1, p + 1)), list(range(p, 0, -1))):
+        wa = engine.strides(list(shape), pia)
+        for q in range(1, p + 1):
+            b = torch.rand(shape[q - 1], generator=g, device=cuda) * 2 - 1
+            nc, pic = engine.output_shape(list(shape), q), engine.output_layout(pia, q)
+            wc = engine.strides(nc, pic)
+            P, nq, S = orc.canonical(list(shape), pia, q)
+            for off in (0, 1, 2):
+                a = buf[off:off + N]
+                c = torch.full((N // nq,), float("nan"), device=cuda)
+                engine.ttv(q, p, a.view(torch.int16), list(shape), wa, pia, b, [nq], c, nc, wc, pic,
+                           dtype=engine.BF16A, sync=True)
+                ref, absn = orc.truth(S, nq, P, a.double().cpu().numpy(), b.double().cpu().numpy())
+                assert orc.rel_error(c.cpu().numpy(), ref, absn) <= 4 * 2.0 ** -24, (pia, q, off)
+            a = buf[:N].clone()
+            a.view(-1)[[0, N // 2, N - 1]] = torch.tensor([float("inf"), float("nan"), float("-inf")],
+                                                          dtype=torch.bfloat16, device=cuda)
+            engine.ttv(q, p, a.view(torch.int16), list(shape), wa, pia, b, [nq], c, nc, wc, pic,
+                       dtype=engine.BF16A, sync=True)
+            bad = ~torch.isfinite(a.view(S, nq, P)).all(dim=1).view(-1)
+            assert torch.equal(~torch.isfinite(c), bad), (pia, q)
+
+
 @pytest.mark.parametrize("dtype", ["f32", "f64", "bf16"])
 @pytest.mark.parametrize("P", [1, 2, 3, 5, 6, 7, 12, 24, 33, 40, 56, 100, 120])
 def test_thin_prefixes_of_any_width(engine, orc, cuda, P, dtype):

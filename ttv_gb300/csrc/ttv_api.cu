@@ -371,12 +371,13 @@ bool default_choices(const tlibg_options* opt)
 int make_plan_inner(int dtype, const Canon& cn, const void* a, const void* b, const tlibg_options* opt,
                     int sms, Plan* out);
 
-// fp32 plans that run faster on the general-stride kernels, which share the
-// contracted mode over warps and clusters without a second kernel and schedule
+// fp32 and bf16 plans that run faster on the general-stride kernels, which share
+// the contracted mode over warps and clusters without a second kernel and schedule
 // many short columns as many CTAs.  Measured against the dense plan on 4 to 256 MB
-// (device time, inputs rotated through L2):
+// (device time, inputs rotated through L2), fp32:
 //   rows split by the plan, A up to 2^26 elements: 1.3 to 2.5 times as fast below
-//     2^24 (512 x 4096: 6.9 -> 2.9 us, 4096 x 4096: 15.9 -> 11.4), level at 2^26;
+//     2^24 (512 x 4096: 6.9 -> 2.9 us, 4096 x 4096: 15.9 -> 11.4), level at 2^26
+//     (rows over 2^16 long slower there: 256 x 262144: 45.8 -> 47.4);
 //   columns split by the plan: 16-byte loads up to 2^25 elements (256^3: 17.5 ->
 //     13.4 us, 2^25: 30 -> 25; 19404 x 1777 above it 29 -> 38), prefixes under 48
 //     up to 2^21 (40 x 5242 x 20: 9.2 -> 10.8), narrower loads up to 2^23 (from
@@ -387,23 +388,41 @@ int make_plan_inner(int dtype, const Canon& cn, const void* a, const void* b, co
 //     slabs of a small A (2 x 2138 x 16: 4.2 -> 5.7);
 //   contractions of at most 4 rows, A of 2^26 elements or more and a prefix of 16
 //     (2^28: 208 -> 197 us, 2^25: level, 2^23: 7.0 -> 8.4; a prefix of 4: 84 -> 112).
+// bf16 (the dense kernels hold 32 to 64 bytes in flight per thread, these 64 and
+// more warps):
+//   rows of 96 elements or more in 16-byte loads (16384 x 4096: 38.7 -> 28.0 us,
+//     500000 x 104: 33.8 -> 30.8; 65536 x 64 level, 1000000 x 64: 40.3 -> 42.4);
+//   rows split by the plan while b stays in L1 or A is small (300000 x 101: 41.9 ->
+//     32.7, 4096 x 1001: 10.1 -> 6.2; 200 rows of 66032: 17.2 -> 19.2);
+//   thin prefixes by the fp32 rule (64^4: 17.0 -> 10.3 us);
+//   columns in loads of two elements or more (6 x 7 x 10^6: 45.0 -> 27.8 us, 512^3:
+//     63 -> 52, 1024^2: 7.2 -> 4.3), one element up to 2^24 (1001 x 100 x 100: 13.4 ->
+//     7.9; 301^3 25.0 -> 27.2, 501 x 7 x 10001: 37.5 -> 74.5).
 // Contractions over more than 2^20 elements keep the fp64 combine.
 void route_general(const Canon& cn, const void* a, const void* b, int sms, Plan* pl)
 {
-    if (pl->dtype != F32 || !pl->kahan || cn.nq > (uint64_t(1) << 20)) return;
+    if (pl->dtype == F64 || !pl->kahan || cn.nq > (uint64_t(1) << 20)) return;
     const uint64_t elems = cn.P * cn.nq * cn.S;
+    const bool bf16 = pl->dtype == BF16A;
     bool take = false;
     if (pl->kind == KIND_ROW) {
-        take = pl->split > 1 && elems <= (uint64_t(1) << 26);
+        if (bf16) {
+            const bool cached_b = cn.nq <= (uint64_t(1) << 15) || elems <= (uint64_t(1) << 22);
+            take = pl->split > 1 ? cached_b : pl->vec == 8 && cn.nq >= 96;
+        } else {
+            take = pl->split > 1 && elems <= (uint64_t(1) << (cn.nq > (uint64_t(1) << 16) ? 25 : 26));
+        }
     } else if (pl->kind == KIND_COL_THIN) {
         take = cn.nq * cn.P <= (uint64_t(1) << 14) &&
                (cn.P >= 8 ? cn.S > (uint64_t)sms || pl->split > 1 : cn.S > (uint64_t)sms && elems <= (uint64_t(1) << 18));
     } else if (pl->kind == KIND_COL) {
-        if (pl->rows_m == 1) take = elems >= (uint64_t(1) << 26) && cn.P >= 16;
+        if (bf16) take = pl->vec >= 2 || elems <= (uint64_t(1) << 24);
+        else if (pl->rows_m == 1) take = elems >= (uint64_t(1) << 26) && cn.P >= 16;
         else take = pl->split > 1 && elems <= (uint64_t(1) << (pl->vec < 4 ? 23 : (cn.P >= 48 ? 25 : 21)));
     }
     if (!take) return;
     GSPlan g;
+    g.dtype = pl->dtype;
     std::vector<std::tuple<size_t, size_t, size_t>> modes;
     if (cn.P > 1) modes.emplace_back(1, cn.P, 1);
     if (cn.S > 1) modes.emplace_back(cn.nq * cn.P, cn.S, cn.P);
@@ -1288,7 +1307,7 @@ int tlibg_ttv_strided(int dtype, size_t q, size_t p, const void* a, const size_t
     pl.k.wb = wb;
     const int sms = dev_info().sms;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    pl.f64 = dtype == F64;
+    pl.dtype = dtype;
     gs_plan(sms, &pl);
     if (pl.k.nseg > 1)
         if (int s = get_scratch(st, gs_partial_bytes(pl), &pl.k.part)) return s;

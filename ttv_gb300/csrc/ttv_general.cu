@@ -14,8 +14,8 @@
 //   row form (q is A's fastest mode): a group of G lanes owns R outputs and
 //     strides over their n_q elements, U loads in flight per output; a shuffle
 //     tree sums the group's lanes in fixed order.
-// V is 16 bytes where the view puts every load on the 16-byte grid, else one
-// element.
+// V is 16 bytes where the view puts every load on the 16-byte grid (bf16 columns
+// on the 4-byte grid: two elements), else one element.
 //
 // Few outputs: the contracted mode is shared by WI warps of a CTA, by the CTAs
 // of a cluster and, beyond that, by segments of the grid.  Warps and CTAs
@@ -24,12 +24,13 @@
 // memory in fixed order, so splitting up to 64 ways costs no second kernel and
 // no scratch.  Segments meet in gs_combine_kernel.
 //
-// Arithmetic: fp32 Kahan; fp64 products rounded once and summed exactly in
+// Arithmetic: fp32 Kahan (bf16-stored A is widened as it is loaded); fp64 products rounded once and summed exactly in
 // 128-bit fixed point (FxAcc), because GB300 issues two FP64 instructions per
 // SM and clock: Kahan's four per element cap a view at 1.2 TB/s, the one
 // multiply left here at 4.7.
 #include "ttv_general.h"
 #include "ttv_device.cuh"
+#include "ttv_kernels.cuh"
 
 #include <cooperative_groups.h>
 
@@ -45,7 +46,8 @@ namespace tlibg {
 // Resident CTAs per SM the kernels are compiled for.  An unshared fp32 kernel
 // lives off warps in flight: 6 for one-element columns (38 x 814,000 outputs:
 // 30.9 us, 42 when the shared form's code held it to 4), 4 for 16-byte columns
-// (5 spills into the loop: 25.2 -> 30.0 us on 33 x 889,000).  The fp64 kernels
+// (5 spills into the loop: 25.2 -> 30.0 us on 33 x 889,000; 3 for bf16 ones: 256 x
+// 1024 x 512 50.6 -> 57.8).  The fp64 kernels
 // hold 128-bit sums: 4 and 3, with the spills outside the loops (2 and 2 were
 // 3 to 30 % slower).
 template <typename T, int N, bool SHARE> constexpr int gs_col_ctas()
@@ -307,24 +309,28 @@ template <int N> struct GsSum<double, N, true> {
 // --------------------------------------------------------------------------
 // 16-byte vectors stream (read once); single elements go through L1, whose
 // sectors serve the neighbours (rows off the 32-byte grid, strided elements).
-template <typename T, int V> __device__ __forceinline__ void gs_load(const T* p, T* out)
+template <typename TA, typename T, int V> __device__ __forceinline__ void gs_load(const TA* p, T* out)
 {
-    if constexpr (V == 1) {
-        out[0] = __ldg(p);
-    } else {
-        T t[V];
-        load_a<T, T, V>(p, t);
+    T t[V];
+    if constexpr (V * sizeof(TA) < 16)
+        load_a_l1<TA, T, V>(p, t);
+    else
+        load_a<TA, T, V>(p, t);
 #pragma unroll
-        for (int v = 0; v < V; ++v) out[v] = t[v];
-    }
+    for (int v = 0; v < V; ++v) out[v] = t[v];
 }
 template <typename T, int V> __device__ __forceinline__ void gs_load_b(const T* p, T* out)
 {
     if constexpr (V == 1) {
         out[0] = __ldg(p);
     } else {
-        const uint4 r = __ldg(reinterpret_cast<const uint4*>(p));
-        memcpy(out, &r, 16);
+        constexpr int W = 16 / (int)sizeof(T);
+        static_assert(V % W == 0, "b in 16-byte loads");
+#pragma unroll
+        for (int w = 0; w < V / W; ++w) {
+            const uint4 r = __ldg(reinterpret_cast<const uint4*>(p) + w);
+            memcpy(out + w * W, &r, 16);
+        }
     }
 }
 
@@ -416,8 +422,8 @@ __device__ __forceinline__ void gs_range(const GSArgs& k, uint64_t seg, uint64_t
 // --------------------------------------------------------------------------
 // U rows, all loads before any product (PART: the column's last `count` < U
 // rows; the loads past them repeat the last row and are not used).
-template <int U, bool PART, typename T, int V, int MO, bool FX>
-__device__ __forceinline__ void gs_col_rows(GsSum<T, MO * V, FX>& sum, const T* (&rp)[MO], uint64_t step, const T*& bp,
+template <int U, bool PART, typename TA, typename T, int V, int MO, bool FX>
+__device__ __forceinline__ void gs_col_rows(GsSum<T, MO * V, FX>& sum, const TA* (&rp)[MO], uint64_t step, const T*& bp,
                                             uint64_t bstep, int count)
 {
     T av[U][MO * V], bv[U][MO * V];
@@ -426,7 +432,7 @@ __device__ __forceinline__ void gs_col_rows(GsSum<T, MO * V, FX>& sum, const T* 
         const T bb = __ldg(bp);
 #pragma unroll
         for (int m = 0; m < MO; ++m) {
-            gs_load<T, V>(rp[m], &av[u][m * V]);
+            gs_load<TA, T, V>(rp[m], &av[u][m * V]);
             if (!PART || u + 1 < count || u + 1 == U) rp[m] += step;
         }
         if (!PART || u + 1 < count || u + 1 == U) bp += bstep;
@@ -436,7 +442,7 @@ __device__ __forceinline__ void gs_col_rows(GsSum<T, MO * V, FX>& sum, const T* 
     sum.template add<PART>(av, bv, count);
 }
 
-template <typename T, int V, int MO, int U, bool FX, bool SHARE>
+template <typename TA, typename T, int V, int MO, int U, bool FX, bool SHARE>
 __global__ void __launch_bounds__(256, gs_col_ctas<T, V * MO, SHARE>()) gs_col_kernel(GSArgs k)
 {
     pdl_prologue();
@@ -462,20 +468,20 @@ __global__ void __launch_bounds__(256, gs_col_ctas<T, V * MO, SHARE>()) gs_col_k
         GsSum<T, N, FX> sum;
         sum.init();
         uint64_t co[MO];
-        const T* rp[MO];
+        const TA* rp[MO];
 #pragma unroll
         for (int m = 0; m < MO; ++m) {
             // one past the end re-reads the tile's first vector (its sums are not stored)
             const uint64_t o = t0 + pos + 32u * V * m;
             uint64_t ao;
             gs_offsets(k, o < k.outputs ? o : t0, ao, co[m]);
-            rp[m] = static_cast<const T*>(k.a) + ao + i * k.waq;
+            rp[m] = static_cast<const TA*>(k.a) + ao + i * k.waq;
         }
         const T* bp = static_cast<const T*>(k.b) + i * k.wb;
         const uint64_t step = k.waq << wl, bstep = k.wb << wl;
-        for (; rows >= U; rows -= U) gs_col_rows<U, false, T, V, MO, FX>(sum, rp, step, bp, bstep, U);
+        for (; rows >= U; rows -= U) gs_col_rows<U, false, TA, T, V, MO, FX>(sum, rp, step, bp, bstep, U);
         for (; rows > 0; rows -= min(rows, (uint64_t)H))
-            gs_col_rows<H, true, T, V, MO, FX>(sum, rp, step, bp, bstep, (int)min(rows, (uint64_t)H));
+            gs_col_rows<H, true, TA, T, V, MO, FX>(sum, rp, step, bp, bstep, (int)min(rows, (uint64_t)H));
         sum.finish();
         if constexpr (!SHARE) {
 #pragma unroll
@@ -508,8 +514,8 @@ __global__ void __launch_bounds__(256, gs_col_ctas<T, V * MO, SHARE>()) gs_col_k
 // --------------------------------------------------------------------------
 // U loads of each of the group's R rows, all before any product.  fp32: a sum
 // per row and vector slot (N = R V); fp64 (exact sums): one per row (N = R).
-template <int U, bool PART, typename T, int V, int R, int N, bool FX>
-__device__ __forceinline__ void gs_row_step(GsSum<T, N, FX>& sum, const T* (&rp)[R], uint64_t step, const T*& bp,
+template <int U, bool PART, typename TA, typename T, int V, int R, int N, bool FX>
+__device__ __forceinline__ void gs_row_step(GsSum<T, N, FX>& sum, const TA* (&rp)[R], uint64_t step, const T*& bp,
                                             uint64_t bstep, int count)
 {
     constexpr int K = N == R ? V : 1;   // vector slots that meet in one sum
@@ -522,7 +528,7 @@ __device__ __forceinline__ void gs_row_step(GsSum<T, N, FX>& sum, const T* (&rp)
 #pragma unroll
         for (int r = 0; r < R; ++r) {
             T t[V];
-            gs_load<T, V>(rp[r], t);
+            gs_load<TA, T, V>(rp[r], t);
             if (!PART || u + 1 < count || u + 1 == U) rp[r] += step;
 #pragma unroll
             for (int v = 0; v < V; ++v) {
@@ -535,7 +541,7 @@ __device__ __forceinline__ void gs_row_step(GsSum<T, N, FX>& sum, const T* (&rp)
     sum.template add<PART>(av, bv, count * K);
 }
 
-template <typename T, int V, int R, int U, bool FX, bool SHARE>
+template <typename TA, typename T, int V, int R, int U, bool FX, bool SHARE>
 __global__ void __launch_bounds__(256, gs_row_ctas<T>()) gs_row_kernel(GSArgs k)
 {
     pdl_prologue();
@@ -561,21 +567,21 @@ __global__ void __launch_bounds__(256, gs_row_ctas<T>()) gs_row_kernel(GSArgs k)
         GsSum<T, N, FX> sum;
         sum.init();
         uint64_t co[R];
-        const T* rp[R];
+        const TA* rp[R];
 #pragma unroll
         for (int r = 0; r < R; ++r) {
             // one past the end re-reads the tile's first row (its sums are not stored)
             const uint64_t o = t0 + r0 + (uint64_t)r * per;
             uint64_t ao;
             gs_offsets(k, o < k.outputs ? o : t0, ao, co[r]);
-            rp[r] = static_cast<const T*>(k.a) + ao + (i0 + first * V) * k.waq;
+            rp[r] = static_cast<const TA*>(k.a) + ao + (i0 + first * V) * k.waq;
         }
         const T* bp = static_cast<const T*>(k.b) + (i0 + first * V) * k.wb;
         const uint64_t step = (V * k.waq) << every, bstep = (V * k.wb) << every;
         uint64_t n = first < nv ? ((nv - first - 1) >> every) + 1 : 0;
-        for (; n >= U; n -= U) gs_row_step<U, false, T, V, R, N, FX>(sum, rp, step, bp, bstep, U);
+        for (; n >= U; n -= U) gs_row_step<U, false, TA, T, V, R, N, FX>(sum, rp, step, bp, bstep, U);
         for (; n > 0; n -= min(n, (uint64_t)H))
-            gs_row_step<H, true, T, V, R, N, FX>(sum, rp, step, bp, bstep, (int)min(n, (uint64_t)H));
+            gs_row_step<H, true, TA, T, V, R, N, FX>(sum, rp, step, bp, bstep, (int)min(n, (uint64_t)H));
         sum.finish();
         Acc<T, true> acc[R];
 #pragma unroll
@@ -675,32 +681,44 @@ typedef void (*GsFn)(GSArgs);
 template <bool SHARE> static GsFn gs_kernel_of(const GSPlan& p, int& U)
 {
     const int M = p.M;
-    if (p.f64) {
+    if (p.dtype == BF16A) {
+        if (p.row) {
+            U = p.V > 1 ? 4 : 8 / M;
+            if (p.V > 1) return gs_row_kernel<uint16_t, float, 8, 1, 4, false, SHARE>;
+            return M == 4 ? gs_row_kernel<uint16_t, float, 1, 4, 2, false, SHARE>
+                          : (M == 2 ? gs_row_kernel<uint16_t, float, 1, 2, 4, false, SHARE> : gs_row_kernel<uint16_t, float, 1, 1, 8, false, SHARE>);
+        }
+        U = p.V == 8 ? 4 : 8;
+        if (p.V == 8) return gs_col_kernel<uint16_t, float, 8, 1, 4, false, SHARE>;
+        if (p.V == 2) return gs_col_kernel<uint16_t, float, 2, 2, 8, false, SHARE>;
+        return M == 2 ? gs_col_kernel<uint16_t, float, 1, 2, 8, false, SHARE> : gs_col_kernel<uint16_t, float, 1, 1, 8, false, SHARE>;
+    }
+    if (p.dtype == F64) {
         if (!p.fx) {   // one element per load and output
             U = 8;
-            return p.row ? gs_row_kernel<double, 1, 1, 8, false, SHARE> : gs_col_kernel<double, 1, 1, 8, false, SHARE>;
+            return p.row ? gs_row_kernel<double, double, 1, 1, 8, false, SHARE> : gs_col_kernel<double, double, 1, 1, 8, false, SHARE>;
         }
         if (p.row) {
             U = p.V > 1 ? 4 / M : 8 / M;
             if (p.V > 1)
-                return M == 4 ? gs_row_kernel<double, 2, 4, 1, true, SHARE>
-                              : (M == 2 ? gs_row_kernel<double, 2, 2, 2, true, SHARE> : gs_row_kernel<double, 2, 1, 4, true, SHARE>);
-            return M == 4 ? gs_row_kernel<double, 1, 4, 2, true, SHARE>
-                          : (M == 2 ? gs_row_kernel<double, 1, 2, 4, true, SHARE> : gs_row_kernel<double, 1, 1, 8, true, SHARE>);
+                return M == 4 ? gs_row_kernel<double, double, 2, 4, 1, true, SHARE>
+                              : (M == 2 ? gs_row_kernel<double, double, 2, 2, 2, true, SHARE> : gs_row_kernel<double, double, 2, 1, 4, true, SHARE>);
+            return M == 4 ? gs_row_kernel<double, double, 1, 4, 2, true, SHARE>
+                          : (M == 2 ? gs_row_kernel<double, double, 1, 2, 4, true, SHARE> : gs_row_kernel<double, double, 1, 1, 8, true, SHARE>);
         }
         U = 4;
-        return p.V > 1 ? gs_col_kernel<double, 2, 1, 4, true, SHARE> : gs_col_kernel<double, 1, 1, 4, true, SHARE>;
+        return p.V > 1 ? gs_col_kernel<double, double, 2, 1, 4, true, SHARE> : gs_col_kernel<double, double, 1, 1, 4, true, SHARE>;
     }
     if (p.row) {
         U = p.V > 1 ? 4 / M : 8 / M;
-        if (p.V > 1) return M == 2 ? gs_row_kernel<float, 4, 2, 2, false, SHARE> : gs_row_kernel<float, 4, 1, 4, false, SHARE>;
-        return M == 4 ? gs_row_kernel<float, 1, 4, 2, false, SHARE>
-                      : (M == 2 ? gs_row_kernel<float, 1, 2, 4, false, SHARE> : gs_row_kernel<float, 1, 1, 8, false, SHARE>);
+        if (p.V > 1) return M == 2 ? gs_row_kernel<float, float, 4, 2, 2, false, SHARE> : gs_row_kernel<float, float, 4, 1, 4, false, SHARE>;
+        return M == 4 ? gs_row_kernel<float, float, 1, 4, 2, false, SHARE>
+                      : (M == 2 ? gs_row_kernel<float, float, 1, 2, 4, false, SHARE> : gs_row_kernel<float, float, 1, 1, 8, false, SHARE>);
     }
     U = p.V > 1 ? 4 / M : (M == 4 ? 4 : 8);
-    if (p.V > 1) return M == 2 ? gs_col_kernel<float, 4, 2, 2, false, SHARE> : gs_col_kernel<float, 4, 1, 4, false, SHARE>;
-    return M == 4 ? gs_col_kernel<float, 1, 4, 4, false, SHARE>
-                  : (M == 2 ? gs_col_kernel<float, 1, 2, 8, false, SHARE> : gs_col_kernel<float, 1, 1, 8, false, SHARE>);
+    if (p.V > 1) return M == 2 ? gs_col_kernel<float, float, 4, 2, 2, false, SHARE> : gs_col_kernel<float, float, 4, 1, 4, false, SHARE>;
+    return M == 4 ? gs_col_kernel<float, float, 1, 4, 4, false, SHARE>
+                  : (M == 2 ? gs_col_kernel<float, float, 1, 2, 8, false, SHARE> : gs_col_kernel<float, float, 1, 1, 8, false, SHARE>);
 }
 static GsFn gs_kernel(const GSPlan& p, bool share, int* u = nullptr)
 {
@@ -748,7 +766,7 @@ static void gs_split(GSPlan* p, uint64_t rows, bool may_split, uint32_t outs_per
         return (k.outputs + to - 1) / to;
     };
     auto up = [](uint64_t a, uint64_t b) { return (a + b - 1) / b; };
-    const double row_clk = 256.0 * N * (p->f64 ? (p->fx ? 0.5 : 2.0) : 4.0 / 23.0);
+    const double row_clk = 256.0 * N * (p->dtype == F64 ? (p->fx ? 0.5 : 2.0) : (p->dtype == BF16A ? 2.0 : 4.0) / 23.0);
     double best = 0;
     uint64_t nseg = 1;
     k.wi_log2 = k.cluster_log2 = 0;
@@ -766,7 +784,7 @@ static void gs_split(GSPlan* p, uint64_t rows, bool may_split, uint32_t outs_per
             // fp64 fixed point: turning a sum into a pair, and FP64 instructions per merge
             const double over = p->fx ? N * (500 + 1024 * (1 - 1.0 / (1 << wl))) : 0;
             const double even = (double)(ctas * ns) / sms;   // HBM serves the SMs alike, the FP64 pipes are their own
-            const double rate = p->f64 ? n * (r * row_clk + over) : std::max(even, 0.4 * n) * r * row_clk;
+            const double rate = p->dtype == F64 ? n * (r * row_clk + over) : std::max(even, 0.4 * n) * r * row_clk;
             const double cost = std::cbrt(rate * rate * rate + chain * chain * chain);
             if ((wl == 0 && cl == 0) || cost < 0.95 * best) {
                 best = cost;
@@ -790,46 +808,56 @@ static void gs_split(GSPlan* p, uint64_t rows, bool may_split, uint32_t outs_per
 void gs_plan(int sms, GSPlan* p)
 {
     GSArgs& k = p->k;
-    const uint64_t V = p->f64 ? 2 : 4;
-    const bool a16 = (reinterpret_cast<uintptr_t>(k.a) % 16) == 0;
+    const bool f64 = p->dtype == F64, bf16 = p->dtype == BF16A;
+    const uint64_t ea = f64 ? 8 : (bf16 ? 2 : 4);
     p->row = k.nm == 0 || (k.nq > 1 && k.waq <= k.wa[0]);
-    bool grid16 = a16;   // every mode but the one loads run along steps in whole vectors
-    for (int r = p->row ? 0 : 1; r < k.nm; ++r) grid16 = grid16 && k.wa[r] % V == 0;
+    // every mode but the one loads run along steps in whole vectors of V elements
+    auto on_grid = [&](uint64_t V) {
+        bool yes = (reinterpret_cast<uintptr_t>(k.a) % (V * ea)) == 0;
+        for (int r = p->row ? 0 : 1; r < k.nm; ++r) yes = yes && k.wa[r] % V == 0;
+        return yes;
+    };
+    const uint64_t V = 16 / ea;
     // fp64: Kahan sums (four FP64 instructions an element against one, but a tenth of
     // the code) while all of them together are about a microsecond of the FP64 pipes
-    p->fx = p->f64 && k.outputs * k.nq > (uint64_t)sms * 1500;
-    const bool plain = p->f64 && !p->fx;
+    p->fx = f64 && k.outputs * k.nq > (uint64_t)sms * 1500;
+    const bool plain = f64 && !p->fx;
     const uint64_t lanes = (uint64_t)sms * 512;
     if (p->row) {
-        p->V = !plain && k.waq == 1 && k.nq % V == 0 && k.wb == 1 && (reinterpret_cast<uintptr_t>(k.b) % 16) == 0 && grid16
+        p->V = !plain && k.waq == 1 && k.nq % V == 0 && k.wb == 1 && (reinterpret_cast<uintptr_t>(k.b) % 16) == 0 && on_grid(V)
                    ? (int)V : 1;
         const uint64_t nv = k.nq / p->V;
         // lanes per output: about eight loads each (fp64, whose sums meet in FP64
         // instructions, 32), and no more lanes than loads
         uint32_t gl = 0;
-        const uint64_t per_lane = p->f64 ? 32 : 8;
-        const uint64_t want = p->f64 ? (uint64_t)sms * 128 : lanes / 2;
+        const uint64_t per_lane = f64 ? 32 : 8;
+        const uint64_t want = f64 ? (uint64_t)sms * 128 : lanes / 2;
         while (gl < 5 && (nv >> (gl + 1)) >= per_lane) ++gl;
-        if (!p->f64 && gl == 0 && nv > 8) gl = 1;
+        if (!f64 && gl == 0 && nv > 8) gl = 1;
         // few outputs: more lanes each, and whole warps before warps share a row
         while (gl < 5 && (k.outputs << gl) < want && (nv >> (gl + 1)) >= 2) ++gl;
         k.group_log2 = gl;
         const uint64_t lane_rows = (nv + (1u << gl) - 1) >> gl;
         // rows per group: several where a row is only a load or two per lane
-        // (16-byte fp32 vectors: two at most, four spill)
-        p->M = plain || lane_rows > 4 ? 1 : (lane_rows > 2 || p->V == 4 ? 2 : 4);
+        // (16-byte fp32 vectors: two at most, four spill; bf16 ones hold eight sums already)
+        p->M = plain || lane_rows > 4 || p->V == 8 ? 1 : (lane_rows > 2 || p->V == 4 ? 2 : 4);
         while (p->M > 1 && (k.outputs << gl) < lanes * p->M) p->M /= 2;
         gs_split(p, lane_rows, gl == 5, (uint32_t)((32u >> gl) * p->M), p->V * p->M, sms);
     } else {
-        p->V = !plain && k.wa[0] == 1 && k.ext[0].d % V == 0 && k.waq % V == 0 && grid16 ? (int)V : 1;
+        auto columns = [&](uint64_t v) { return k.wa[0] == 1 && k.ext[0].d % v == 0 && k.waq % v == 0 && on_grid(v); };
+        p->V = !plain && columns(V) ? (int)V : 1;
         // 16-byte vectors only while they leave a warp on every scheduler: the
         // contracted mode is shared 64 ways at most before the grid is split
         if (p->V > 1 && k.outputs / V * std::min<uint64_t>(64, std::max<uint64_t>(1, k.nq / 8)) < lanes / 2) p->V = 1;
-        // single elements: two outputs per thread, four in short columns, one where
-        // there are too few to fill the chip
-        if (p->V > 1) p->M = !p->f64 && k.nq <= 4 && k.outputs / (2 * V) >= lanes * 2 ? 2 : 1;
-        else if (k.nq <= 4 && !p->f64 && k.outputs / 4 >= lanes * 2) p->M = 4;
-        else p->M = !p->f64 && k.nq >= 64 && k.outputs >= lanes ? 2 : 1;
+        if (bf16 && p->V == 1 && columns(2)) {
+            p->V = p->M = 2;   // 4-byte loads, two vectors per thread
+        } else if (p->V > 1) {
+            p->M = p->dtype == F32 && k.nq <= 4 && k.outputs / (2 * V) >= lanes * 2 ? 2 : 1;
+        } else if (k.nq <= 4 && p->dtype == F32 && k.outputs / 4 >= lanes * 2) {
+            p->M = 4;   // single elements: four outputs per thread in short columns,
+        } else {        // two in long ones, one where there are too few to fill the chip
+            p->M = !f64 && k.nq >= 64 && k.outputs >= lanes ? 2 : 1;
+        }
         gs_split(p, k.nq, true, (uint32_t)(32 * p->V * p->M), p->V * p->M, sms);
     }
 }
@@ -860,7 +888,7 @@ cudaError_t gs_launch(const GSPlan& p, cudaStream_t st, int sms, uint64_t* launc
         attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
         attr[0].val.programmaticStreamSerializationAllowed = 1;
         cfg.numAttrs = 1;
-        e = cudaLaunchKernelEx(&cfg, p.f64 ? gs_combine_kernel<double> : gs_combine_kernel<float>, p.k);
+        e = cudaLaunchKernelEx(&cfg, p.dtype == F64 ? gs_combine_kernel<double> : gs_combine_kernel<float>, p.k);
         if (e != cudaSuccess) return e;
         ++*launches;
     }

@@ -36,7 +36,8 @@ struct GSArgs {
 
 struct GSPlan {
     GSArgs k{};
-    bool f64 = false, row = false;
+    int dtype = 0;          // element types, numbered as the plan's (fp32, fp64, bf16-stored A)
+    bool row = false;
     bool fx = false;        // fp64: fixed-point sums (else Kahan)
     int V = 1, M = 1;       // vector width; vectors per thread (column) or rows per group (row)
     int grid = 1;
@@ -55,7 +56,7 @@ cudaError_t gs_launch(const GSPlan& p, cudaStream_t st, int sms, uint64_t* launc
 // Bytes of partial sums the plan needs (args.part), 0 without segments.
 inline size_t gs_partial_bytes(const GSPlan& p)
 {
-    return p.k.nseg > 1 ? (size_t)p.k.nseg * p.k.outputs * 2 * (p.f64 ? 8 : 4) : 0;
+    return p.k.nseg > 1 ? (size_t)p.k.nseg * p.k.outputs * 2 * (p.dtype == 1 ? 8 : 4) : 0;
 }
 
 }  // namespace tlibg
