@@ -909,6 +909,25 @@ def test_bf16_plans_on_the_general_stride_kernels(engine, orc, cuda, shape):
             assert torch.equal(~torch.isfinite(c), bad), (pia, q)
 
 
+@pytest.mark.parametrize("dtype", ["f32", "f64"])
+def test_row_shift_zeros_in_b(engine, cuda, dtype):
+    """Row-shift kernel with zeros (of both signs) among b's elements: small whole numbers, so every
+    sum is exact and compared bit for bit."""
+    import torch
+    g = torch.Generator(device=cuda)
+    g.manual_seed(3)
+    tdt = torch.float64 if dtype == "f64" else torch.float32
+    for nq, S in ((125, 5), (65, 300), (645, 40), (1001, 9)):
+        a = torch.randint(-9, 10, (S, nq), generator=g, device=cuda).to(tdt)
+        b = torch.randint(-2, 3, (nq,), generator=g, device=cuda).to(tdt)
+        b[::7] = -0.0
+        for G in (2, 8, 32):
+            c = torch.full((S,), float("nan"), device=cuda, dtype=tdt)
+            engine.ttv(1, 2, a, [nq, S], [1, nq], [1, 2], b, [nq], c, [S, 1], [1, S], [1, 2],
+                       kind=engine.KIND_ROW_SHIFT, group=G, sync=True)
+            assert torch.equal(c, (a.double() @ b.double()).to(tdt)), (nq, S, G)
+
+
 @pytest.mark.parametrize("dtype", ["f32", "f64", "bf16"])
 @pytest.mark.parametrize("P", [1, 2, 3, 5, 6, 7, 12, 24, 33, 40, 56, 100, 120])
 def test_thin_prefixes_of_any_width(engine, orc, cuda, P, dtype):
