@@ -929,6 +929,40 @@ def test_row_shift_zeros_in_b(engine, cuda, dtype):
 
 
 @pytest.mark.parametrize("dtype", ["f32", "f64", "bf16"])
+@pytest.mark.parametrize("nq", [64, 65, 66, 71, 102, 255, 257, 258, 511, 513, 645, 1023, 1025, 1281, 1535, 2001])
+def test_rows_off_the_vector_grid(engine, orc, cuda, nq, dtype):
+    """q-fastest rows of every misalignment around the lines between the row, row-shift and
+    general-stride kernels: one row to several rounds of lane groups, A on and off the 16-byte
+    grid, infinities and NaN in the first, a middle and the last row.  Bars: fp32 and bf16 storage
+    4 x 2^-24 of sum |a b|; fp64 the suite's 1e-13."""
+    import torch
+    g = torch.Generator(device=cuda)
+    g.manual_seed(nq)
+    dt = {"f32": engine.F32, "f64": engine.F64, "bf16": engine.BF16A}[dtype]
+    tdt = torch.float64 if dtype == "f64" else torch.float32
+    for S in (1, 2, 37, 255, 256, 1000, 9727, 9728, 10001, 20001):
+        N = nq * S
+        buf = torch.rand(N + 7, generator=g, device=cuda, dtype=tdt) * 2 - 1
+        if dtype == "bf16":
+            buf = buf.to(torch.bfloat16)
+        b = torch.rand(nq, generator=g, device=cuda, dtype=tdt) * 2 - 1
+        for off in ((0, 1, 3, 6) if S < 300 else (0, 1)):
+            a = buf[off:off + N]
+            c = torch.full((S,), float("nan"), device=cuda, dtype=tdt)
+            call = lambda: engine.ttv(1, 2, a.view(torch.int16) if dtype == "bf16" else a, [nq, S], [1, nq], [1, 2], b,
+                                      [nq], c, [S, 1], [1, S], [1, 2], dtype=dt, sync=True)
+            call()
+            rows, bd = a.view(S, nq).double(), b.double()
+            ref, absn = rows @ bd, rows.abs() @ bd.abs()
+            err = ((c.double() - ref).abs() / absn).max().item()
+            assert err <= (1e-13 if dtype == "f64" else 4 * 2.0 ** -24), (S, off, err)
+        for r, bad in ((0, "inf"), (S // 2, "nan"), (S - 1, "-inf")):
+            a.view(S, nq)[r, (r * 7) % nq] = float(bad)
+        call()
+        assert torch.equal(torch.isfinite(c), torch.isfinite(a.view(S, nq)).all(dim=1)), S
+
+
+@pytest.mark.parametrize("dtype", ["f32", "f64", "bf16"])
 @pytest.mark.parametrize("P", [1, 2, 3, 5, 6, 7, 12, 24, 33, 40, 56, 100, 120])
 def test_thin_prefixes_of_any_width(engine, orc, cuda, P, dtype):
     """Thin prefixes whose vectors divide the warp and not (idle lanes), one to several slabs,

@@ -574,8 +574,7 @@ int make_row_panel_plan(Plan pl, const Canon& cn, const tlibg_options* opt, int 
 }
 
 // Rows that are not whole 16-byte vectors: the row-shift kernel (aligned
-// vector bodies against shifted copies of b in shared memory), G lanes per row
-// by the row kernel's rule, no split.
+// vector bodies against shifted copies of b in shared memory), no split.
 int make_row_shift_plan(Plan pl, const Canon& cn, const tlibg_options* opt, int sms, Plan* out)
 {
     const int vmax = (int)(16 / elem_size_a(pl.dtype));
@@ -583,11 +582,14 @@ int make_row_shift_plan(Plan pl, const Canon& cn, const tlibg_options* opt, int 
         return fail(TLIBG_ERR_ARGUMENT, "tlibg: the row-shift kernel loads 16 bytes per vector");
     if (opt && opt->split > 1)
         return fail(TLIBG_ERR_ARGUMENT, "tlibg: the row-shift kernel does not split the contracted mode");
-    int G;
-    if (pl.dtype == F64)
-        G = std::max(2, std::min(32, pow2_floor(std::max<uint64_t>(1, cn.nq / 64))));
-    else
-        G = std::max(2, std::min(32, pow2_floor(std::max<uint64_t>(1, cn.nq / 4 / 16))));
+    // Lanes per row: 32 elements each (fp64 and bf16 64), 8 lanes at most, 16 for rows
+    // over 1280 (fp32 501 x 134000: 8 lanes 49.1 us, 4 50.7, 16 52.8; fp64 255 x 263000:
+    // 4 lanes 99.5, 2 104, 8 105); with few rows more, until the lanes fill the GPU
+    // once (fp64 645 x 400: 32 lanes 5.2 us, 8 8.9)
+    const bool f64 = pl.dtype == F64;
+    const uint64_t per_lane = pl.dtype == F32 ? 32 : 64;
+    int G = std::max(2, std::min(cn.nq > 1280 ? 16 : 8, pow2_floor(std::max<uint64_t>(1, (cn.nq + 1) / per_lane))));
+    while (G < 32 && cn.S * G < (uint64_t)sms * (f64 ? 460 : 425)) G *= 2;
     if (opt && opt->group > 0) G = opt->group;
     if (G < 1 || G > 32 || (G & (G - 1)))
         return fail(TLIBG_ERR_ARGUMENT, "tlibg: lanes per row must be a power of two in 1..32");
@@ -657,10 +659,9 @@ int make_plan_inner(int dtype, const Canon& cn, const void* a, const void* b, co
                                             "than one segment of b");
         return make_row_panel_plan(pl, cn, opt, sms, out);
     }
-    const bool shift_ok = cn.P == 1 && dtype != BF16A &&
-                          rs_smem_bytes(cn.nq, et, dtype == F64 && pl.kahan) <= RS_SMEM_MAX;
+    const bool shift_ok = cn.P == 1 && rs_smem_bytes(dtype, cn.nq, pl.kahan) <= RS_SMEM_MAX;
     if (opt && opt->kind == KIND_ROW_SHIFT) {
-        if (!shift_ok)
+        if (!shift_ok || dtype == BF16A)
             return fail(TLIBG_ERR_ARGUMENT, "tlibg: the row-shift kernel needs prefix P == 1, fp32 or fp64 A, "
                                             "and b's shifted copies within 48 KB of shared memory");
         return make_row_shift_plan(pl, cn, opt, sms, out);
@@ -696,19 +697,32 @@ int make_plan_inner(int dtype, const Canon& cn, const void* a, const void* b, co
         return make_stream_plan(pl, cn, opt, sms, out);
     }
     // Rows of 64 or more elements that are not whole 16-byte vectors (or A off the
-    // 16-byte grid), with enough rows to fill the lane groups without a split: the
-    // row-shift kernel instead of the row kernel's scalar loads (measured on GB300
-    // for the sweep's rows of 645 floats / doubles).
-    if (shift_ok && !rows_aligned && cn.nq >= 64 && no_split && !(opt && (opt->kind >= 0 || opt->vec > 0))) {
-        Plan sp;
-        if (make_row_shift_plan(pl, cn, opt, sms, &sp) == TLIBG_OK) {
-            // at least four rounds of rows over the resident lane groups (the kernel
-            // has no split to fill the GPU with fewer rows)
-            const uint64_t groups = (uint64_t)sms * std::max(1, plan_ctas_per_sm(sp)) * (BLOCK / sp.group);
-            if (cn.S >= 4 * groups) {
-                *out = sp;
-                return TLIBG_OK;
-            }
+    // 16-byte grid): the row-shift kernel instead of the row kernel's narrow loads.
+    //   fp32: rows enough to pay for the copies of b, 16 per resident CTA (255 x 131586:
+    //     36.6 -> 26.3 us, 1001 x 67041: 59.6 -> 46.9; 1001 x 8380 level, 645 x 3251 3.6
+    //     on the general-stride kernels against 4.6);
+    //   fp64: all but short stacks of long rows (no second kernel: 501 x 523: 7.2 -> 5.3 us,
+    //     255 x 263172: 136 -> 99, 65 x 8: 4.5 -> 3.0; 1001 x 8 level); rows that would
+    //     leave a second round of lane groups under half full stay with the row kernel
+    //     where that needs no split (645 x 26011: 29.5, here 31.7);
+    //   bf16: as fp32, rows of odd length and of 4-byte alignment from 256 elements
+    //     (255 x 263172: 99 -> 37 us, 274 x 200000: 42 -> 30; 102 x 600000: 43.8 -> 47),
+    //     up to 1024 (the eight copies of b take 32 bytes per element).
+    Plan shift;
+    bool shift_last = false;
+    if (shift_ok && !rows_aligned && cn.nq >= 64 && no_split && !(opt && (opt->kind >= 0 || opt->vec > 0)) &&
+        make_row_shift_plan(pl, cn, opt, sms, &shift) == TLIBG_OK) {
+        const uint64_t ctas = (uint64_t)sms * std::max(1, plan_ctas_per_sm(shift));
+        const uint64_t groups = ctas * (BLOCK / shift.group);
+        bool take;
+        if (opt && opt->group > 0) take = dtype != BF16A && cn.S >= 4 * groups;
+        else if (dtype == F64) take = cn.nq <= 512 || cn.S >= 256;
+        else take = cn.S >= 16 * ctas &&
+                    (dtype == F32 || (cn.nq <= 1024 && (cn.nq % 2 || (cn.nq % 4 && cn.nq >= 256))));
+        shift_last = take && dtype == F64 && cn.S > groups && 2 * cn.S < 3 * groups;
+        if (take && !shift_last) {
+            *out = shift;
+            return TLIBG_OK;
         }
     }
     const int vmax = (int)(16 / ea);
@@ -795,6 +809,10 @@ int make_plan_inner(int dtype, const Canon& cn, const void* a, const void* b, co
                     nseg = ns;
         }
         nseg = std::max<uint64_t>(1, std::min<uint64_t>(nseg, cn.nq));
+        if (shift_last && nseg > 1) {
+            *out = shift;
+            return TLIBG_OK;
+        }
         uint64_t seg_len = cdiv(cn.nq, nseg);
         seg_len = cdiv(seg_len, V) * V;
         nseg = cdiv(cn.nq, seg_len);

@@ -92,11 +92,11 @@ struct Plan {
 // splits for fp64 with the mix; at most RS_SMEM_MAX bytes.
 constexpr size_t RS_SMEM_MAX = 48 * 1024;
 __host__ __device__ inline uint64_t rs_width(uint64_t nq, int V) { return (nq + V + V - 1) / V * V; }
-__host__ __device__ inline size_t rs_smem_bytes(uint64_t nq, size_t es, bool split)
+inline size_t rs_smem_bytes(int dtype, uint64_t nq, bool kahan)
 {
-    const int V = (int)(16 / es);
-    const uint64_t W = rs_width(nq, V);
-    return (size_t)V * W * es + (split ? (size_t)V * W * 8 : 0);
+    const int V = dtype == F64 ? 2 : (dtype == BF16A ? 8 : 4);
+    const size_t copies = (size_t)V * rs_width(nq, V);
+    return copies * (dtype == F64 ? 8 : 4) + (dtype == F64 && kahan ? copies * 8 : 0);
 }
 
 // Whether the streamed kernel can take a problem (whole rows fit a stage).

@@ -13,9 +13,14 @@
 // aligned vector bsh[m][x0 + kV..] with x0 = 0 (m == 0) or V.  fp64 with the
 // double-float mix keeps the copies' splits beside them.
 //
-//   items        rows, G lanes each (the row kernel's lane rule), no split
-//   per lane     body vectors gl, gl + G, ... with U loads in flight; head and
-//                tail elements gl < count
+// bf16-stored A: V = 8, so eight fp32 copies of b and two 16-byte shared loads per
+// vector; U = 2 in 64 registers (U = 4 in 77: 36.3 us on 645 x 104044, this 35.1).
+//
+//   items        rows, G lanes each, no split
+//   per lane     body vectors gl, gl + G, ... with U loads in flight, U / 2 of the
+//                rest together (645 x 104044 fp64: 97.1 -> 95.6 us with them; one
+//                masked block of U - 1 instead: fp32 44.9 -> 51.2); head and tail
+//                elements gl < count
 //   output       the G lanes' sums meet in a warp shuffle tree (fixed order)
 //
 // Shared memory: V W elements of b (+ V W float2 for the fp64 mix), at most
@@ -24,22 +29,33 @@
 
 namespace tlibg {
 
-template <typename T, bool KAHAN>
+// V elements of a shifted copy of b.
+template <int V, typename T> __device__ __forceinline__ void rs_load_b(const T* p, T (&out)[V])
+{
+    typedef typename RawVec<16>::type R;
+    constexpr int W = 16 / (int)sizeof(T);
+#pragma unroll
+    for (int w = 0; w < V / W; ++w) {
+        const R r = *(reinterpret_cast<const R*>(p) + w);
+        memcpy(out + w * W, &r, 16);
+    }
+}
+
+template <typename TA, typename T, bool KAHAN>
 __global__ void __launch_bounds__(BLOCK, 4) row_shift_kernel(KArgs k)
 {
     pdl_prologue();
-    constexpr int V = 16 / (int)sizeof(T);
-    constexpr int U = 4;
+    constexpr int V = 16 / (int)sizeof(TA);
+    constexpr int U = sizeof(TA) == 2 ? 2 : 4;
     constexpr bool PRES = presplit_b<T, KAHAN>();
     typedef typename AccSel<T, KAHAN>::type AccT;
-    typedef typename RawVec<16>::type R;
     extern __shared__ __align__(128) unsigned char smem_raw[];
     const uint64_t nq = k.nq;
     const uint32_t W = (uint32_t)rs_width(nq, V);
     T* bsh = reinterpret_cast<T*>(smem_raw);
     float2* bsp = reinterpret_cast<float2*>(smem_raw + (size_t)V * W * sizeof(T));
     const T* __restrict__ B = static_cast<const T*>(k.b);
-    const T* __restrict__ A = static_cast<const T*>(k.a);
+    const TA* __restrict__ A = static_cast<const TA*>(k.a);
 
     int ok = 1;
     for (uint32_t idx = threadIdx.x; idx < (uint32_t)V * W; idx += BLOCK) {
@@ -66,7 +82,7 @@ __global__ void __launch_bounds__(BLOCK, 4) row_shift_kernel(KArgs k)
     const uint32_t gpw = 32u / G;
     const uint64_t warp_id = (uint64_t(blockIdx.x) * BLOCK + threadIdx.x) >> 5;
     const uint64_t nwarps = (uint64_t(gridDim.x) * BLOCK) >> 5;
-    const uintptr_t abase = reinterpret_cast<uintptr_t>(A) / sizeof(T);   // element address of A
+    const uintptr_t abase = reinterpret_cast<uintptr_t>(A) / sizeof(TA);   // element address of A
 
     for (uint64_t wbase = warp_id * gpw; wbase < k.items; wbase += nwarps * gpw) {
         const uint64_t row = wbase + lane / G;
@@ -79,45 +95,45 @@ __global__ void __launch_bounds__(BLOCK, 4) row_shift_kernel(KArgs k)
             const uint64_t head = min((uint64_t)((V - m) & (V - 1)), nq);
             const uint64_t nvb = (nq - head) / V;            // body vectors
             const uint64_t tail0 = head + nvb * V;           // first tail element (row position)
-            const T* ab = A + rs + head;                     // 16-byte aligned
+            const TA* ab = A + rs + head;                    // 16-byte aligned
             const uint32_t x0 = m == 0 ? 0u : (uint32_t)V;
             const T* bb = bsh + (size_t)m * W + x0;
             const float2* bp = bsp + (size_t)m * W + x0;
-            uint64_t kv = gl;
-            for (; kv + (U - 1) * G < nvb; kv += U * G) {
-                T av[U][V], bv[U][V];
-#pragma unroll
-                for (int u = 0; u < U; ++u) {
-                    load_a<T, T, V>(ab + (kv + u * G) * V, av[u]);
-                    const R r = *reinterpret_cast<const R*>(bb + (kv + u * G) * V);
-                    memcpy(bv[u], &r, 16);
-                }
-#pragma unroll
-                for (int u = 0; u < U; ++u) {
-                    if constexpr (PRES) {
-                        if (pre_ok)
-                            vec_fma<V, true>(acc, av[u], bv[u], u, bp + (kv + u * G) * V);
-                        else
-                            vec_fma<V, false>(acc, av[u], bv[u], u);
-                    } else {
-                        vec_fma<V, false>(acc, av[u], bv[u], u);
-                    }
-                }
-                renorm_all<V>(acc);
-            }
-            for (; kv < nvb; kv += G) {
-                T av[1][V], bv[1][V];
-                load_a<T, T, V>(ab + kv * V, av[0]);
-                const R r = *reinterpret_cast<const R*>(bb + kv * V);
-                memcpy(bv[0], &r, 16);
+            auto add = [&](const T (&av)[V], int u, uint64_t kv) {
+                T bv[V];
+                rs_load_b<V, T>(bb + kv * V, bv);
                 if constexpr (PRES) {
                     if (pre_ok)
-                        vec_fma<V, true>(acc, av[0], bv[0], 0, bp + kv * V);
+                        vec_fma<V, true>(acc, av, bv, u, bp + kv * V);
                     else
-                        vec_fma<V, false>(acc, av[0], bv[0], 0);
+                        vec_fma<V, false>(acc, av, bv, u);
                 } else {
-                    vec_fma<V, false>(acc, av[0], bv[0], 0);
+                    vec_fma<V, false>(acc, av, bv, u);
                 }
+            };
+            uint64_t kv = gl;
+            for (; kv + (U - 1) * G < nvb; kv += U * G) {
+                T av[U][V];
+#pragma unroll
+                for (int u = 0; u < U; ++u) load_a<TA, T, V>(ab + (kv + u * G) * V, av[u]);
+#pragma unroll
+                for (int u = 0; u < U; ++u) add(av[u], u, kv + u * G);
+                renorm_all<V>(acc);
+            }
+            if constexpr (U > 2) {
+                if (kv + (U / 2 - 1) * G < nvb) {
+                    T av[U / 2][V];
+#pragma unroll
+                    for (int u = 0; u < U / 2; ++u) load_a<TA, T, V>(ab + (kv + u * G) * V, av[u]);
+#pragma unroll
+                    for (int u = 0; u < U / 2; ++u) add(av[u], u, kv + u * G);
+                    kv += U / 2 * G;
+                }
+            }
+            for (; kv < nvb; kv += G) {
+                T av[V];
+                load_a<TA, T, V>(ab + kv * V, av);
+                add(av, 0, kv);
             }
             renorm_all<V>(acc);
             // head [0, head) and tail [tail0, nq): b in place (copy 0)
@@ -125,7 +141,7 @@ __global__ void __launch_bounds__(BLOCK, 4) row_shift_kernel(KArgs k)
             for (uint64_t t = gl; t < head + nt; t += G) {
                 const uint64_t e = t < head ? t : tail0 + (t - head);
                 T av[1];
-                load_a<T, T, 1>(A + rs + e, av);
+                load_a<TA, T, 1>(A + rs + e, av);
                 acc[0].fma_add(av[0], bsh[e]);
             }
         }
