@@ -378,6 +378,9 @@ int make_plan_inner(int dtype, const Canon& cn, const void* a, const void* b, co
 //   rows split by the plan, A up to 2^26 elements: 1.3 to 2.5 times as fast below
 //     2^24 (512 x 4096: 6.9 -> 2.9 us, 4096 x 4096: 15.9 -> 11.4), level at 2^26
 //     (rows over 2^16 long slower there: 256 x 262144: 45.8 -> 47.4);
+//   unsplit rows of a multiple of 64 elements in 16-byte loads, whose lanes all take
+//     whole blocks of loads (2097152 x 128: 164 -> 157 us, 349525 x 192: 47.4 -> 42.0,
+//     131072 x 512: 42.2 -> 41.0; of 100, 144 and 320 level or 5 % slower);
 //   columns split by the plan: 16-byte loads up to 2^25 elements (256^3: 17.5 ->
 //     13.4 us, 2^25: 30 -> 25; 19404 x 1777 above it 29 -> 38), prefixes under 48
 //     up to 2^21 (40 x 5242 x 20: 9.2 -> 10.8), narrower loads up to 2^23 (from
@@ -410,7 +413,8 @@ void route_general(const Canon& cn, const void* a, const void* b, int sms, Plan*
             const bool cached_b = cn.nq <= (uint64_t(1) << 15) || elems <= (uint64_t(1) << 22);
             take = pl->split > 1 ? cached_b : pl->vec == 8 && cn.nq >= 96;
         } else {
-            take = pl->split > 1 && elems <= (uint64_t(1) << (cn.nq > (uint64_t(1) << 16) ? 25 : 26));
+            take = pl->split > 1 ? elems <= (uint64_t(1) << (cn.nq > (uint64_t(1) << 16) ? 25 : 26))
+                                 : pl->vec == 4 && cn.nq % 64 == 0;
         }
     } else if (pl->kind == KIND_COL_THIN) {
         take = cn.nq * cn.P <= (uint64_t(1) << 14) &&
