@@ -929,7 +929,8 @@ def test_row_shift_zeros_in_b(engine, cuda, dtype):
 
 
 @pytest.mark.parametrize("dtype", ["f32", "f64", "bf16"])
-@pytest.mark.parametrize("nq", [64, 65, 66, 71, 102, 255, 257, 258, 511, 513, 645, 1023, 1025, 1281, 1535, 2001])
+@pytest.mark.parametrize("nq", [34, 64, 65, 66, 71, 102, 255, 256, 257, 258, 511, 513, 514, 645, 1023, 1024, 1025, 1281, 1500,
+                                1534, 1535, 2001])
 def test_rows_off_the_vector_grid(engine, orc, cuda, nq, dtype):
     """q-fastest rows of every misalignment around the lines between the row, row-shift and
     general-stride kernels: one row to several rounds of lane groups, A on and off the 16-byte
@@ -940,7 +941,7 @@ def test_rows_off_the_vector_grid(engine, orc, cuda, nq, dtype):
     g.manual_seed(nq)
     dt = {"f32": engine.F32, "f64": engine.F64, "bf16": engine.BF16A}[dtype]
     tdt = torch.float64 if dtype == "f64" else torch.float32
-    for S in (1, 2, 37, 255, 256, 1000, 9727, 9728, 10001, 20001):
+    for S in (1, 2, 37, 255, 256, 511, 512, 1000, 9727, 9728, 10001, 20001):
         N = nq * S
         buf = torch.rand(N + 7, generator=g, device=cuda, dtype=tdt) * 2 - 1
         if dtype == "bf16":

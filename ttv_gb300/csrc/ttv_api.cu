@@ -587,12 +587,14 @@ int make_row_shift_plan(Plan pl, const Canon& cn, const tlibg_options* opt, int 
     if (opt && opt->split > 1)
         return fail(TLIBG_ERR_ARGUMENT, "tlibg: the row-shift kernel does not split the contracted mode");
     // Lanes per row: 32 elements each (fp64 and bf16 64), 8 lanes at most, 16 for rows
-    // over 1280 (fp32 501 x 134000: 8 lanes 49.1 us, 4 50.7, 16 52.8; fp64 255 x 263000:
+    // over 1280 in more than one round (fp64 1401 x 44000: 97 -> 90 us, 1500 x 10000 32 ->
+    // 36; fp32 501 x 134000: 8 lanes 49.1 us, 4 50.7, 16 52.8; fp64 255 x 263000:
     // 4 lanes 99.5, 2 104, 8 105); with few rows more, until the lanes fill the GPU
     // once (fp64 645 x 400: 32 lanes 5.2 us, 8 8.9)
     const bool f64 = pl.dtype == F64;
     const uint64_t per_lane = pl.dtype == F32 ? 32 : 64;
-    int G = std::max(2, std::min(cn.nq > 1280 ? 16 : 8, pow2_floor(std::max<uint64_t>(1, (cn.nq + 1) / per_lane))));
+    const int most = cn.nq > 1280 && cn.S > (uint64_t)sms * 128 ? 16 : 8;
+    int G = std::max(2, std::min(most, pow2_floor(std::max<uint64_t>(1, (cn.nq + 1) / per_lane))));
     while (G < 32 && cn.S * G < (uint64_t)sms * (f64 ? 460 : 425)) G *= 2;
     if (opt && opt->group > 0) G = opt->group;
     if (G < 1 || G > 32 || (G & (G - 1)))
@@ -706,24 +708,26 @@ int make_plan_inner(int dtype, const Canon& cn, const void* a, const void* b, co
     //     36.6 -> 26.3 us, 1001 x 67041: 59.6 -> 46.9; 1001 x 8380 level, 645 x 3251 3.6
     //     on the general-stride kernels against 4.6);
     //   fp64: all but short stacks of long rows (no second kernel: 501 x 523: 7.2 -> 5.3 us,
-    //     255 x 263172: 136 -> 99, 65 x 8: 4.5 -> 3.0; 1001 x 8 level); rows that would
-    //     leave a second round of lane groups under half full stay with the row kernel
-    //     where that needs no split (645 x 26011: 29.5, here 31.7);
+    //     255 x 263172: 136 -> 99, 65 x 8: 4.5 -> 3.0; 1001 x 8 level), rows on the grid
+    //     too where the row kernel would split them (over 64 long: 128 x 30000: 15.6 -> 9.1 us,
+    //     512 x 1000: 6.4 -> 4.3, 1024 x 100000: 147 -> 134, 100 x 8: 4.8 -> 3.3; level
+    //     where it would not); rows off it that would leave a second round of lane groups under
+    //     half full also stay with the unsplit row kernel (645 x 26011: 29.5, here 31.7);
     //   bf16: as fp32, rows of odd length and of 4-byte alignment from 256 elements
     //     (255 x 263172: 99 -> 37 us, 274 x 200000: 42 -> 30; 102 x 600000: 43.8 -> 47),
     //     up to 1024 (the eight copies of b take 32 bytes per element).
     Plan shift;
     bool shift_last = false;
-    if (shift_ok && !rows_aligned && cn.nq >= 64 && no_split && !(opt && (opt->kind >= 0 || opt->vec > 0)) &&
+    if (shift_ok && (rows_aligned ? dtype == F64 && pl.kahan && cn.nq > 64 : cn.nq >= 64) && no_split && !(opt && (opt->kind >= 0 || opt->vec > 0)) &&
         make_row_shift_plan(pl, cn, opt, sms, &shift) == TLIBG_OK) {
         const uint64_t ctas = (uint64_t)sms * std::max(1, plan_ctas_per_sm(shift));
         const uint64_t groups = ctas * (BLOCK / shift.group);
         bool take;
-        if (opt && opt->group > 0) take = dtype != BF16A && cn.S >= 4 * groups;
-        else if (dtype == F64) take = cn.nq <= 512 || cn.S >= 256;
+        if (opt && opt->group > 0) take = !rows_aligned && dtype != BF16A && cn.S >= 4 * groups;
+        else if (dtype == F64) take = cn.nq <= 512 || cn.S >= (rows_aligned ? 512 : 256);
         else take = cn.S >= 16 * ctas &&
                     (dtype == F32 || (cn.nq <= 1024 && (cn.nq % 2 || (cn.nq % 4 && cn.nq >= 256))));
-        shift_last = take && dtype == F64 && cn.S > groups && 2 * cn.S < 3 * groups;
+        shift_last = take && dtype == F64 && (rows_aligned || (cn.S > groups && 2 * cn.S < 3 * groups));
         if (take && !shift_last) {
             *out = shift;
             return TLIBG_OK;
