@@ -928,6 +928,44 @@ def test_row_shift_zeros_in_b(engine, cuda, dtype):
             assert torch.equal(c, (a.double() @ b.double()).to(tdt)), (nq, S, G)
 
 
+@pytest.mark.parametrize("shape", [(64, 64, 64), (261, 589), (31, 100, 300), (4096, 250), (128, 63, 128), (20, 30, 40), (5, 5, 5),
+                                   (1024, 4096), (4100, 3070), (40, 3000), (16, 400, 16), (2, 9, 3000), (301, 7, 1991),
+                                   (25, 100, 5000), (512, 8, 1030), (16, 9, 58300)], ids=lambda s: "x".join(map(str, s)))
+def test_fp64_plans_on_the_general_stride_kernels(engine, orc, cuda, shape):
+    """fp64 calls around the same lines: shared and unshared columns in 16-byte and single loads,
+    rows, thin prefixes, A on and off the 16-byte grid, elements outside the double-float window
+    (tiny, huge, zero), infinities and NaN.  Bar: the suite's 1e-13 of sum |a b|."""
+    import torch
+    g = torch.Generator(device=cuda)
+    g.manual_seed(int(np.prod(shape)) % 100003)
+    p, N = len(shape), int(np.prod(shape))
+    buf = torch.rand(N + 1, generator=g, device=cuda, dtype=torch.float64) * 2 - 1
+    buf[::17] *= 2.0 ** -300
+    buf[::29] = 0.0
+    for pia in (list(range(1, p + 1)), list(range(p, 0, -1))):
+        wa = engine.strides(list(shape), pia)
+        for q in range(1, p + 1):
+            b = torch.rand(shape[q - 1], generator=g, device=cuda, dtype=torch.float64) * 2 - 1
+            b[::3] = 0.0
+            nc, pic = engine.output_shape(list(shape), q), engine.output_layout(pia, q)
+            wc = engine.strides(nc, pic)
+            P, nq, S = orc.canonical(list(shape), pia, q)
+            for off in (0, 1):
+                a = buf[off:off + N]
+                c = torch.full((N // nq,), float("nan"), device=cuda, dtype=torch.float64)
+                call = lambda t: engine.ttv(q, p, t, list(shape), wa, pia, b, [nq], c, nc, wc, pic, sync=True)
+                call(a)
+                t = a.view(S, nq, P)
+                ref = torch.einsum("sip,i->sp", t, b).reshape(-1)
+                absn = torch.einsum("sip,i->sp", t.abs(), b.abs()).reshape(-1)
+                assert ((c - ref).abs() <= 1e-13 * absn + 1e-300).all(), (pia, q, off)
+            a = buf[:N].clone()
+            a[[0, N // 2, N - 1]] = torch.tensor([float("inf"), float("nan"), float("-inf")], dtype=torch.float64, device=cuda)
+            b[b == 0] = 0.5
+            call(a)
+            assert torch.equal(torch.isfinite(c), torch.isfinite(a.view(S, nq, P)).all(dim=1).reshape(-1)), (pia, q)
+
+
 @pytest.mark.parametrize("dtype", ["f32", "f64", "bf16"])
 @pytest.mark.parametrize("nq", [34, 64, 65, 66, 71, 102, 255, 256, 257, 258, 511, 513, 514, 645, 1023, 1024, 1025, 1281, 1500,
                                 1534, 1535, 2001])

@@ -371,7 +371,7 @@ bool default_choices(const tlibg_options* opt)
 int make_plan_inner(int dtype, const Canon& cn, const void* a, const void* b, const tlibg_options* opt,
                     int sms, Plan* out);
 
-// fp32 and bf16 plans that run faster on the general-stride kernels, which share
+// Plans that run faster on the general-stride kernels, which share
 // the contracted mode over warps and clusters without a second kernel and schedule
 // many short columns as many CTAs.  Measured against the dense plan on 4 to 256 MB
 // (device time, inputs rotated through L2), fp32:
@@ -401,21 +401,34 @@ int make_plan_inner(int dtype, const Canon& cn, const void* a, const void* b, co
 //   columns in loads of two elements or more (6 x 7 x 10^6: 45.0 -> 27.8 us, 512^3:
 //     63 -> 52, 1024^2: 7.2 -> 4.3), one element up to 2^24 (1001 x 100 x 100: 13.4 ->
 //     7.9; 301^3 25.0 -> 27.2, 501 x 7 x 10001: 37.5 -> 74.5).
-// Contractions over more than 2^20 elements keep the fp64 combine.
+// fp64 (the dense kernels' mixed products, no second launch), without segments of
+// the grid (16 x 10000: 6.6 -> 9.2):
+//   rows that the plan splits, up to 3 x 2^22 elements (1024 x 4096: 18.3 -> 10.6 us,
+//     4000 x 2001: 23.2 -> 17.1; 4096 x 4096: 30.5 -> 35.2), others up to 2^21;
+//   columns in 16-byte loads up to 2^26 elements where warps share the contraction or
+//     it is at most 8 long (256^3: 33.3 -> 27.9, 128^3: 8.3 -> 6.0, 1024^2: 7.4 -> 5.3;
+//     512^3: 168.6 -> 171.9), else 2^23 (8 x 16 x 100000: 22.0 -> 22.3);
+//   columns in single loads up to 2^24 elements, of under 64 rows 2^22 (31 x 100 x
+//     3000: 26.2 -> 18.7; 645 x 645 x 64: 51 -> 59, 301 x 7 x 3000: 18.0 -> 22.6).
+// Contractions over more than 2^20 elements keep the dense kernels' combine.
 void route_general(const Canon& cn, const void* a, const void* b, int sms, Plan* pl)
 {
-    if (pl->dtype == F64 || !pl->kahan || cn.nq > (uint64_t(1) << 20)) return;
+    if (!pl->kahan || cn.nq > (uint64_t(1) << 20)) return;
     const uint64_t elems = cn.P * cn.nq * cn.S;
-    const bool bf16 = pl->dtype == BF16A;
+    const bool bf16 = pl->dtype == BF16A, f64 = pl->dtype == F64;
     bool take = false;
     if (pl->kind == KIND_ROW) {
-        if (bf16) {
+        if (f64) {
+            take = elems <= (pl->split > 1 ? uint64_t(3) << 22 : uint64_t(1) << 21);
+        } else if (bf16) {
             const bool cached_b = cn.nq <= (uint64_t(1) << 15) || elems <= (uint64_t(1) << 22);
             take = pl->split > 1 ? cached_b : pl->vec == 8 && cn.nq >= 96;
         } else {
             take = pl->split > 1 ? elems <= (uint64_t(1) << (cn.nq > (uint64_t(1) << 16) ? 25 : 26))
                                  : pl->vec == 4 && cn.nq % 64 == 0;
         }
+    } else if (f64) {   // and, below, by the plan's vectors and sharing
+        take = (pl->kind == KIND_COL_THIN || pl->kind == KIND_COL) && elems <= (uint64_t(1) << 26);
     } else if (pl->kind == KIND_COL_THIN) {
         take = cn.nq * cn.P <= (uint64_t(1) << 14) &&
                (cn.P >= 8 ? cn.S > (uint64_t)sms || pl->split > 1 : cn.S > (uint64_t)sms && elems <= (uint64_t(1) << 18));
@@ -426,6 +439,7 @@ void route_general(const Canon& cn, const void* a, const void* b, int sms, Plan*
     }
     if (!take) return;
     GSPlan g;
+    g.mix = f64;
     g.dtype = pl->dtype;
     std::vector<std::tuple<size_t, size_t, size_t>> modes;
     if (cn.P > 1) modes.emplace_back(1, cn.P, 1);
@@ -437,6 +451,11 @@ void route_general(const Canon& cn, const void* a, const void* b, int sms, Plan*
     g.k.waq = cn.nq > 1 ? cn.P : 0;
     g.k.wb = 1;
     gs_plan(sms, &g);
+    if (f64) {
+        if (g.k.nseg > 1) return;
+        const uint64_t most = g.V == 2 ? (g.k.wi_log2 || cn.nq <= 8 ? 26 : 23) : (cn.nq >= 64 ? 24 : 22);
+        if (!g.row && elems > (uint64_t(1) << most)) return;
+    }
     pl->general = true;
     pl->kind = g.row ? KIND_ROW : KIND_COL;
     pl->rows_m = 0;

@@ -176,6 +176,17 @@ __device__ __forceinline__ DSplit split_double(double x)
     return r;
 }
 
+// The same to the nearest of the 47 bits kept (a carry may pass into the exponent):
+// for b where its split serves several products.  Against truncating both factors
+// the products' error falls by 0.6.
+__device__ __forceinline__ DSplit split_double_nearest(double x)
+{
+    uint32_t hi32 = (uint32_t)__double2hiint(x), lo32 = (uint32_t)__double2loint(x);
+    asm("add.cc.u32 %0, %0, 32;\n\taddc.u32 %1, %1, 0;" : "+r"(lo32), "+r"(hi32));
+    DSplit r = split_double(__hiloint2double((int)hi32, (int)lo32));
+    return r;
+}
+
 // Out-of-window products: a real call, so the compiler cannot turn the rare
 // branch into a predicated DFMA that would take an FP64 issue slot for every
 // in-window product as well.

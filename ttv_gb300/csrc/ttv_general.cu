@@ -187,8 +187,9 @@ __device__ __noinline__ double2 fx_fold(uint4 w, int base, double s, double c)
     return make_double2(a.s, a.c);
 }
 
-// Sums of one thread: N outputs, Kahan or (FX) fixed point.
-template <typename T, int N, bool FX> struct GsSum {
+// Sums of one thread: N outputs, Kahan, fixed point, or (GS_MIX, dense fp64 plans)
+// the dense kernels' mix of native and double-float products.
+template <typename T, int N, int SUM> struct GsSum {
     Acc<T, true> acc[N];
     __device__ __forceinline__ void init()
     {
@@ -210,7 +211,7 @@ template <typename T, int N, bool FX> struct GsSum {
     __device__ __forceinline__ Acc<T, true> get(int n) const { return acc[n]; }
 };
 
-template <int N> struct GsSum<double, N, true> {
+template <int N> struct GsSum<double, N, GS_FX> {
     FxAcc acc[N];
     int base, budget;
     __device__ __forceinline__ void init()
@@ -303,6 +304,44 @@ template <int N> struct GsSum<double, N, true> {
         return a;
     }
 };
+template <int N> struct GsSum<double, N, GS_MIX> {
+    AccDF acc[N];
+    __device__ __forceinline__ void init()
+    {
+#pragma unroll
+        for (int n = 0; n < N; ++n) acc[n].init();
+    }
+    template <bool PART, int UB>
+    __device__ __forceinline__ void add(const double (&x)[UB][N], const double (&y)[UB][N], int count)
+    {
+        static_assert(UB <= 8, "renormalised every 8 products");
+#pragma unroll
+        for (int u = 0; u < UB; ++u) {
+            if (PART && u >= count) break;
+#pragma unroll
+            for (int n = 0; n < N; ++n) {
+                if ((u + n) % 2 == 0)
+                    acc[n].d = fma(x[u][n], y[u][n], acc[n].d);
+                else
+                    acc[n].add_split(split_double(x[u][n]), split_double_nearest(y[u][n]), x[u][n], y[u][n]);
+            }
+        }
+#pragma unroll
+        for (int n = 0; n < N; ++n) acc[n].renorm();
+    }
+    __device__ __forceinline__ void finish()
+    {
+#pragma unroll
+        for (int n = 0; n < N; ++n) acc[n].fold();
+    }
+    __device__ __forceinline__ Acc<double, true> get(int n) const
+    {
+        Acc<double, true> a;
+        a.s = acc[n].s;
+        a.c = 0.0;
+        return a;
+    }
+};
 
 // --------------------------------------------------------------------------
 // loads
@@ -337,6 +376,16 @@ template <typename T, int V> __device__ __forceinline__ void gs_load_b(const T* 
 // --------------------------------------------------------------------------
 // results of a tile: straight to C, or through the warps and the cluster
 // --------------------------------------------------------------------------
+// Another thread's sum into this one's: mixed sums carry no compensation, one
+// addition as in the dense kernels (Kahan's merge is six FP64 instructions).
+template <int SUM, typename T> __device__ __forceinline__ void gs_merge(Acc<T, true>& a, T s, T c)
+{
+    if constexpr (SUM == GS_MIX)
+        a.s += s;
+    else
+        a.merge(s, c);
+}
+
 template <typename T> struct GsPair {
     T s, c;
 };
@@ -357,7 +406,7 @@ __device__ __forceinline__ void gs_put(const GSArgs& k, uint64_t seg, uint64_t o
 // Adds up the tile's slots (slot = position of the output in the tile, first
 // output t0) over the CTA's warp rows, then over the cluster's CTAs, which
 // share the slots; all in fixed order.  red[warp row][slot] in every CTA.
-template <typename T>
+template <typename T, int SUM>
 __device__ __forceinline__ void gs_reduce(const GSArgs& k, GsPair<T>* red, uint32_t slots, uint64_t seg, uint64_t t0)
 {
     namespace cg = cooperative_groups;
@@ -368,7 +417,7 @@ __device__ __forceinline__ void gs_reduce(const GSArgs& k, GsPair<T>* red, uint3
         Acc<T, true> a;
         a.s = src[s].s;
         a.c = src[s].c;
-        for (uint32_t w = 1; w < wi; ++w) a.merge(src[w * slots + s].s, src[w * slots + s].c);
+        for (uint32_t w = 1; w < wi; ++w) gs_merge<SUM>(a, src[w * slots + s].s, src[w * slots + s].c);
         return a;
     };
     __syncthreads();
@@ -400,7 +449,7 @@ __device__ __forceinline__ void gs_reduce(const GSArgs& k, GsPair<T>* red, uint3
         a.c = p[0].c;
 #pragma unroll
         for (int r = 1; r < GS_MAX_CLUSTER; ++r)
-            if ((uint32_t)r < ncta) a.merge(p[r].s, p[r].c);
+            if ((uint32_t)r < ncta) gs_merge<SUM>(a, p[r].s, p[r].c);
         uint64_t ao, co;
         gs_offsets(k, t0 + s, ao, co);
         gs_put<T, true>(k, seg, t0 + s, co, a);
@@ -422,8 +471,8 @@ __device__ __forceinline__ void gs_range(const GSArgs& k, uint64_t seg, uint64_t
 // --------------------------------------------------------------------------
 // U rows, all loads before any product (PART: the column's last `count` < U
 // rows; the loads past them repeat the last row and are not used).
-template <int U, bool PART, typename TA, typename T, int V, int MO, bool FX>
-__device__ __forceinline__ void gs_col_rows(GsSum<T, MO * V, FX>& sum, const TA* (&rp)[MO], uint64_t step, const T*& bp,
+template <int U, bool PART, typename TA, typename T, int V, int MO, int SUM>
+__device__ __forceinline__ void gs_col_rows(GsSum<T, MO * V, SUM>& sum, const TA* (&rp)[MO], uint64_t step, const T*& bp,
                                             uint64_t bstep, int count)
 {
     T av[U][MO * V], bv[U][MO * V];
@@ -442,7 +491,7 @@ __device__ __forceinline__ void gs_col_rows(GsSum<T, MO * V, FX>& sum, const TA*
     sum.template add<PART>(av, bv, count);
 }
 
-template <typename TA, typename T, int V, int MO, int U, bool FX, bool SHARE>
+template <typename TA, typename T, int V, int MO, int U, int SUM, bool SHARE>
 __global__ void __launch_bounds__(256, gs_col_ctas<T, V * MO, SHARE>()) gs_col_kernel(GSArgs k)
 {
     pdl_prologue();
@@ -465,7 +514,7 @@ __global__ void __launch_bounds__(256, gs_col_ctas<T, V * MO, SHARE>()) gs_col_k
             i = i0 + wi;
             rows = i < i1 ? ((i1 - i - 1) >> wl) + 1 : 0;
         }
-        GsSum<T, N, FX> sum;
+        GsSum<T, N, SUM> sum;
         sum.init();
         uint64_t co[MO];
         const TA* rp[MO];
@@ -479,9 +528,9 @@ __global__ void __launch_bounds__(256, gs_col_ctas<T, V * MO, SHARE>()) gs_col_k
         }
         const T* bp = static_cast<const T*>(k.b) + i * k.wb;
         const uint64_t step = k.waq << wl, bstep = k.wb << wl;
-        for (; rows >= U; rows -= U) gs_col_rows<U, false, TA, T, V, MO, FX>(sum, rp, step, bp, bstep, U);
+        for (; rows >= U; rows -= U) gs_col_rows<U, false, TA, T, V, MO, SUM>(sum, rp, step, bp, bstep, U);
         for (; rows > 0; rows -= min(rows, (uint64_t)H))
-            gs_col_rows<H, true, TA, T, V, MO, FX>(sum, rp, step, bp, bstep, (int)min(rows, (uint64_t)H));
+            gs_col_rows<H, true, TA, T, V, MO, SUM>(sum, rp, step, bp, bstep, (int)min(rows, (uint64_t)H));
         sum.finish();
         if constexpr (!SHARE) {
 #pragma unroll
@@ -504,7 +553,7 @@ __global__ void __launch_bounds__(256, gs_col_ctas<T, V * MO, SHARE>()) gs_col_k
                     p.c = a.c;
                     red[wi * TO + pos + 32u * V * m + v] = p;
                 }
-            gs_reduce<T>(k, red, TO, seg, t0);
+            gs_reduce<T, SUM>(k, red, TO, seg, t0);
         }
     }
 }
@@ -514,8 +563,8 @@ __global__ void __launch_bounds__(256, gs_col_ctas<T, V * MO, SHARE>()) gs_col_k
 // --------------------------------------------------------------------------
 // U loads of each of the group's R rows, all before any product.  fp32: a sum
 // per row and vector slot (N = R V); fp64 (exact sums): one per row (N = R).
-template <int U, bool PART, typename TA, typename T, int V, int R, int N, bool FX>
-__device__ __forceinline__ void gs_row_step(GsSum<T, N, FX>& sum, const TA* (&rp)[R], uint64_t step, const T*& bp,
+template <int U, bool PART, typename TA, typename T, int V, int R, int N, int SUM>
+__device__ __forceinline__ void gs_row_step(GsSum<T, N, SUM>& sum, const TA* (&rp)[R], uint64_t step, const T*& bp,
                                             uint64_t bstep, int count)
 {
     constexpr int K = N == R ? V : 1;   // vector slots that meet in one sum
@@ -541,11 +590,11 @@ __device__ __forceinline__ void gs_row_step(GsSum<T, N, FX>& sum, const TA* (&rp
     sum.template add<PART>(av, bv, count * K);
 }
 
-template <typename TA, typename T, int V, int R, int U, bool FX, bool SHARE>
+template <typename TA, typename T, int V, int R, int U, int SUM, bool SHARE>
 __global__ void __launch_bounds__(256, gs_row_ctas<T>()) gs_row_kernel(GSArgs k)
 {
     pdl_prologue();
-    constexpr int N = FX ? R : R * V;
+    constexpr int N = SUM == GS_FX ? R : R * V;
     constexpr int NV = N / R;   // sums per row
     constexpr int H = U > 1 ? U / 2 : 1;   // loads of a masked block at the end
     __shared__ GsPair<T> red[SHARE ? 8 * 32 * R : 1];
@@ -564,7 +613,7 @@ __global__ void __launch_bounds__(256, gs_row_ctas<T>()) gs_row_kernel(GSArgs k)
         if (SHARE) gs_range(k, seg, i0, i1);
         const uint64_t nv = (i1 - i0) / V;   // V divides every range
         const uint64_t first = ((uint64_t)wi << k.group_log2) + gl;   // the lane's first vector of the range
-        GsSum<T, N, FX> sum;
+        GsSum<T, N, SUM> sum;
         sum.init();
         uint64_t co[R];
         const TA* rp[R];
@@ -579,9 +628,9 @@ __global__ void __launch_bounds__(256, gs_row_ctas<T>()) gs_row_kernel(GSArgs k)
         const T* bp = static_cast<const T*>(k.b) + (i0 + first * V) * k.wb;
         const uint64_t step = (V * k.waq) << every, bstep = (V * k.wb) << every;
         uint64_t n = first < nv ? ((nv - first - 1) >> every) + 1 : 0;
-        for (; n >= U; n -= U) gs_row_step<U, false, TA, T, V, R, N, FX>(sum, rp, step, bp, bstep, U);
+        for (; n >= U; n -= U) gs_row_step<U, false, TA, T, V, R, N, SUM>(sum, rp, step, bp, bstep, U);
         for (; n > 0; n -= min(n, (uint64_t)H))
-            gs_row_step<H, true, TA, T, V, R, N, FX>(sum, rp, step, bp, bstep, (int)min(n, (uint64_t)H));
+            gs_row_step<H, true, TA, T, V, R, N, SUM>(sum, rp, step, bp, bstep, (int)min(n, (uint64_t)H));
         sum.finish();
         Acc<T, true> acc[R];
 #pragma unroll
@@ -590,7 +639,7 @@ __global__ void __launch_bounds__(256, gs_row_ctas<T>()) gs_row_kernel(GSArgs k)
 #pragma unroll
             for (int v = 1; v < NV; ++v) {
                 const Acc<T, true> x = sum.get(r * NV + v);
-                acc[r].merge(x.s, x.c);
+                gs_merge<SUM>(acc[r], x.s, x.c);
             }
         }
         for (uint32_t off = (1u << k.group_log2) >> 1; off > 0; off >>= 1) {
@@ -598,7 +647,7 @@ __global__ void __launch_bounds__(256, gs_row_ctas<T>()) gs_row_kernel(GSArgs k)
             for (int r = 0; r < R; ++r) {
                 const T os = __shfl_xor_sync(0xffffffffu, acc[r].s, off);
                 const T oc = __shfl_xor_sync(0xffffffffu, acc[r].c, off);
-                acc[r].merge(os, oc);
+                gs_merge<SUM>(acc[r], os, oc);
             }
         }
         if constexpr (!SHARE) {
@@ -619,7 +668,7 @@ __global__ void __launch_bounds__(256, gs_row_ctas<T>()) gs_row_kernel(GSArgs k)
                     red[wi * TO + r * per + r0] = p;
                 }
             }
-            gs_reduce<T>(k, red, TO, seg, t0);
+            gs_reduce<T, SUM>(k, red, TO, seg, t0);
         }
     }
 }
@@ -684,41 +733,47 @@ template <bool SHARE> static GsFn gs_kernel_of(const GSPlan& p, int& U)
     if (p.dtype == BF16A) {
         if (p.row) {
             U = p.V > 1 ? 4 : 8 / M;
-            if (p.V > 1) return gs_row_kernel<uint16_t, float, 8, 1, 4, false, SHARE>;
-            return M == 4 ? gs_row_kernel<uint16_t, float, 1, 4, 2, false, SHARE>
-                          : (M == 2 ? gs_row_kernel<uint16_t, float, 1, 2, 4, false, SHARE> : gs_row_kernel<uint16_t, float, 1, 1, 8, false, SHARE>);
+            if (p.V > 1) return gs_row_kernel<uint16_t, float, 8, 1, 4, GS_KAHAN, SHARE>;
+            return M == 4 ? gs_row_kernel<uint16_t, float, 1, 4, 2, GS_KAHAN, SHARE>
+                          : (M == 2 ? gs_row_kernel<uint16_t, float, 1, 2, 4, GS_KAHAN, SHARE> : gs_row_kernel<uint16_t, float, 1, 1, 8, GS_KAHAN, SHARE>);
         }
         U = p.V == 8 ? 4 : 8;
-        if (p.V == 8) return gs_col_kernel<uint16_t, float, 8, 1, 4, false, SHARE>;
-        if (p.V == 2) return gs_col_kernel<uint16_t, float, 2, 2, 8, false, SHARE>;
-        return M == 2 ? gs_col_kernel<uint16_t, float, 1, 2, 8, false, SHARE> : gs_col_kernel<uint16_t, float, 1, 1, 8, false, SHARE>;
+        if (p.V == 8) return gs_col_kernel<uint16_t, float, 8, 1, 4, GS_KAHAN, SHARE>;
+        if (p.V == 2) return gs_col_kernel<uint16_t, float, 2, 2, 8, GS_KAHAN, SHARE>;
+        return M == 2 ? gs_col_kernel<uint16_t, float, 1, 2, 8, GS_KAHAN, SHARE> : gs_col_kernel<uint16_t, float, 1, 1, 8, GS_KAHAN, SHARE>;
+    }
+    if (p.dtype == F64 && p.mix) {
+        U = p.V > 1 ? 4 : 8;
+        if (p.row)
+            return p.V > 1 ? gs_row_kernel<double, double, 2, 1, 4, GS_MIX, SHARE> : gs_row_kernel<double, double, 1, 1, 8, GS_MIX, SHARE>;
+        return p.V > 1 ? gs_col_kernel<double, double, 2, 1, 4, GS_MIX, SHARE> : gs_col_kernel<double, double, 1, 1, 8, GS_MIX, SHARE>;
     }
     if (p.dtype == F64) {
         if (!p.fx) {   // one element per load and output
             U = 8;
-            return p.row ? gs_row_kernel<double, double, 1, 1, 8, false, SHARE> : gs_col_kernel<double, double, 1, 1, 8, false, SHARE>;
+            return p.row ? gs_row_kernel<double, double, 1, 1, 8, GS_KAHAN, SHARE> : gs_col_kernel<double, double, 1, 1, 8, GS_KAHAN, SHARE>;
         }
         if (p.row) {
             U = p.V > 1 ? 4 / M : 8 / M;
             if (p.V > 1)
-                return M == 4 ? gs_row_kernel<double, double, 2, 4, 1, true, SHARE>
-                              : (M == 2 ? gs_row_kernel<double, double, 2, 2, 2, true, SHARE> : gs_row_kernel<double, double, 2, 1, 4, true, SHARE>);
-            return M == 4 ? gs_row_kernel<double, double, 1, 4, 2, true, SHARE>
-                          : (M == 2 ? gs_row_kernel<double, double, 1, 2, 4, true, SHARE> : gs_row_kernel<double, double, 1, 1, 8, true, SHARE>);
+                return M == 4 ? gs_row_kernel<double, double, 2, 4, 1, GS_FX, SHARE>
+                              : (M == 2 ? gs_row_kernel<double, double, 2, 2, 2, GS_FX, SHARE> : gs_row_kernel<double, double, 2, 1, 4, GS_FX, SHARE>);
+            return M == 4 ? gs_row_kernel<double, double, 1, 4, 2, GS_FX, SHARE>
+                          : (M == 2 ? gs_row_kernel<double, double, 1, 2, 4, GS_FX, SHARE> : gs_row_kernel<double, double, 1, 1, 8, GS_FX, SHARE>);
         }
         U = 4;
-        return p.V > 1 ? gs_col_kernel<double, double, 2, 1, 4, true, SHARE> : gs_col_kernel<double, double, 1, 1, 4, true, SHARE>;
+        return p.V > 1 ? gs_col_kernel<double, double, 2, 1, 4, GS_FX, SHARE> : gs_col_kernel<double, double, 1, 1, 4, GS_FX, SHARE>;
     }
     if (p.row) {
         U = p.V > 1 ? 4 / M : 8 / M;
-        if (p.V > 1) return M == 2 ? gs_row_kernel<float, float, 4, 2, 2, false, SHARE> : gs_row_kernel<float, float, 4, 1, 4, false, SHARE>;
-        return M == 4 ? gs_row_kernel<float, float, 1, 4, 2, false, SHARE>
-                      : (M == 2 ? gs_row_kernel<float, float, 1, 2, 4, false, SHARE> : gs_row_kernel<float, float, 1, 1, 8, false, SHARE>);
+        if (p.V > 1) return M == 2 ? gs_row_kernel<float, float, 4, 2, 2, GS_KAHAN, SHARE> : gs_row_kernel<float, float, 4, 1, 4, GS_KAHAN, SHARE>;
+        return M == 4 ? gs_row_kernel<float, float, 1, 4, 2, GS_KAHAN, SHARE>
+                      : (M == 2 ? gs_row_kernel<float, float, 1, 2, 4, GS_KAHAN, SHARE> : gs_row_kernel<float, float, 1, 1, 8, GS_KAHAN, SHARE>);
     }
     U = p.V > 1 ? 4 / M : (M == 4 ? 4 : 8);
-    if (p.V > 1) return M == 2 ? gs_col_kernel<float, float, 4, 2, 2, false, SHARE> : gs_col_kernel<float, float, 4, 1, 4, false, SHARE>;
-    return M == 4 ? gs_col_kernel<float, float, 1, 4, 4, false, SHARE>
-                  : (M == 2 ? gs_col_kernel<float, float, 1, 2, 8, false, SHARE> : gs_col_kernel<float, float, 1, 1, 8, false, SHARE>);
+    if (p.V > 1) return M == 2 ? gs_col_kernel<float, float, 4, 2, 2, GS_KAHAN, SHARE> : gs_col_kernel<float, float, 4, 1, 4, GS_KAHAN, SHARE>;
+    return M == 4 ? gs_col_kernel<float, float, 1, 4, 4, GS_KAHAN, SHARE>
+                  : (M == 2 ? gs_col_kernel<float, float, 1, 2, 8, GS_KAHAN, SHARE> : gs_col_kernel<float, float, 1, 1, 8, GS_KAHAN, SHARE>);
 }
 static GsFn gs_kernel(const GSPlan& p, bool share, int* u = nullptr)
 {
@@ -766,7 +821,7 @@ static void gs_split(GSPlan* p, uint64_t rows, bool may_split, uint32_t outs_per
         return (k.outputs + to - 1) / to;
     };
     auto up = [](uint64_t a, uint64_t b) { return (a + b - 1) / b; };
-    const double row_clk = 256.0 * N * (p->dtype == F64 ? (p->fx ? 0.5 : 2.0) : (p->dtype == BF16A ? 2.0 : 4.0) / 23.0);
+    const double row_clk = 256.0 * N * (p->dtype == F64 ? (p->mix ? 0.4 : p->fx ? 0.5 : 2.0) : (p->dtype == BF16A ? 2.0 : 4.0) / 23.0);
     double best = 0;
     uint64_t nseg = 1;
     k.wi_log2 = k.cluster_log2 = 0;
@@ -778,13 +833,13 @@ static void gs_split(GSPlan* p, uint64_t rows, bool may_split, uint32_t outs_per
             if (wl == 3 && cl == 3 && ctas < cap) ns = std::max<uint64_t>(1, std::min<uint64_t>(cap / ctas, rows / (64 * 16)));
             const uint64_t ways = (uint64_t)(1u << (wl + cl)) * ns;
             if (ways > 1 && (!may_split || rows < 2 * ways)) continue;
-            const double fixed = 1500 + (wl ? 5000 : 0) + (cl ? 6000 : 0) + (ns > 1 ? 6000 : 0);
+            const double fixed = 1500 + (wl ? (p->mix ? 3000 : 5000) : 0) + (cl ? (p->mix ? 5000 : 6000) : 0) + (ns > 1 ? 6000 : 0);
             const double n = (double)up(ctas * ns, (uint64_t)sms), r = (double)up(rows, ways);
             const double chain = std::ceil(n / cps) * (std::ceil(r / U) * 1400 + fixed);
             // fp64 fixed point: turning a sum into a pair, and FP64 instructions per merge
             const double over = p->fx ? N * (500 + 1024 * (1 - 1.0 / (1 << wl))) : 0;
             const double even = (double)(ctas * ns) / sms;   // HBM serves the SMs alike, the FP64 pipes are their own
-            const double rate = p->dtype == F64 ? n * (r * row_clk + over) : std::max(even, 0.4 * n) * r * row_clk;
+            const double rate = p->dtype == F64 && !p->mix ? n * (r * row_clk + over) : std::max(even, 0.4 * n) * r * row_clk;
             const double cost = std::cbrt(rate * rate * rate + chain * chain * chain);
             if ((wl == 0 && cl == 0) || cost < 0.95 * best) {
                 best = cost;
@@ -820,8 +875,8 @@ void gs_plan(int sms, GSPlan* p)
     const uint64_t V = 16 / ea;
     // fp64: Kahan sums (four FP64 instructions an element against one, but a tenth of
     // the code) while all of them together are about a microsecond of the FP64 pipes
-    p->fx = f64 && k.outputs * k.nq > (uint64_t)sms * 1500;
-    const bool plain = f64 && !p->fx;
+    p->fx = f64 && !p->mix && k.outputs * k.nq > (uint64_t)sms * 1500;
+    const bool plain = f64 && !p->mix && !p->fx;
     const uint64_t lanes = (uint64_t)sms * 512;
     if (p->row) {
         p->V = !plain && k.waq == 1 && k.nq % V == 0 && k.wb == 1 && (reinterpret_cast<uintptr_t>(k.b) % 16) == 0 && on_grid(V)
@@ -840,7 +895,7 @@ void gs_plan(int sms, GSPlan* p)
         const uint64_t lane_rows = (nv + (1u << gl) - 1) >> gl;
         // rows per group: several where a row is only a load or two per lane
         // (16-byte fp32 vectors: two at most, four spill; bf16 ones hold eight sums already)
-        p->M = plain || lane_rows > 4 || p->V == 8 ? 1 : (lane_rows > 2 || p->V == 4 ? 2 : 4);
+        p->M = plain || p->mix || lane_rows > 4 || p->V == 8 ? 1 : (lane_rows > 2 || p->V == 4 ? 2 : 4);
         while (p->M > 1 && (k.outputs << gl) < lanes * p->M) p->M /= 2;
         gs_split(p, lane_rows, gl == 5, (uint32_t)((32u >> gl) * p->M), p->V * p->M, sms);
     } else {

@@ -34,11 +34,15 @@ struct GSArgs {
     uint32_t group_log2;          // row form: lanes per output
 };
 
+// How a thread sums: Kahan, fp64 products in fixed point, fp64 native and double-float products.
+enum GsMode { GS_KAHAN = 0, GS_FX = 1, GS_MIX = 2 };
+
 struct GSPlan {
     GSArgs k{};
     int dtype = 0;          // element types, numbered as the plan's (fp32, fp64, bf16-stored A)
     bool row = false;
     bool fx = false;        // fp64: fixed-point sums (else Kahan)
+    bool mix = false;       // fp64, set by the caller: the dense kernels' mixed products instead
     int V = 1, M = 1;       // vector width; vectors per thread (column) or rows per group (row)
     int grid = 1;
 };

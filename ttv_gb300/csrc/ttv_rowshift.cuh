@@ -64,7 +64,7 @@ __global__ void __launch_bounds__(BLOCK, 4) row_shift_kernel(KArgs k)
         bsh[idx] = v;
         if constexpr (PRES) {
             // the split of zero (outside its window) is not zero: written out
-            const DSplit d = split_double((double)v);
+            const DSplit d = split_double_nearest((double)v);
             bsp[idx] = v == T(0) ? make_float2(0.0f, 0.0f) : make_float2(d.hi, d.lo);
             ok &= (d.ok || v == T(0)) ? 1 : 0;
         }
