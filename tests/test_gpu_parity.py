@@ -966,6 +966,34 @@ def test_fp64_plans_on_the_general_stride_kernels(engine, orc, cuda, shape):
             assert torch.equal(torch.isfinite(c), torch.isfinite(a.view(S, nq, P)).all(dim=1).reshape(-1)), (pia, q)
 
 
+@pytest.mark.parametrize("dtype", ["f32", "bf16"])
+@pytest.mark.parametrize("nq", [1, 2, 3, 4, 7, 33])
+def test_packed_sums_are_the_scalar_steps(engine, cuda, nq, dtype):
+    """Columns summed by one warp row take Kahan's steps in order: equal bit for bit to the steps in
+    numpy (the fused product in fp64: exact but for a double rounding once in 2^29)."""
+    import torch
+    g = torch.Generator(device=cuda)
+    g.manual_seed(nq)
+    dt = engine.F32 if dtype == "f32" else engine.BF16A
+    for P, opts in ((1032, dict(kind=engine.KIND_COL, group=1, split=1)), (1 << 20, {})):
+        if not opts and nq > 4:
+            continue
+        a = torch.rand(nq, P, generator=g, device=cuda) * 2 - 1
+        a = a if dtype == "f32" else a.to(torch.bfloat16)
+        b = torch.rand(nq, generator=g, device=cuda) * 2 - 1
+        c = torch.full((P,), float("nan"), device=cuda)
+        engine.ttv(2, 2, a if dtype == "f32" else a.view(torch.int16), [P, nq], [1, P], [1, 2], b, [nq], c, [P, 1], [1, P],
+                   [1, 2], dtype=dt, sync=True, **opts)
+        x, y, f = a.float().cpu().numpy(), b.cpu().numpy(), np.float32
+        s, e = np.zeros(P, f), np.zeros(P, f)
+        for i in range(nq):
+            m = (x[i].astype(np.float64) * np.float64(y[i]) - e).astype(f)
+            t = s + m
+            e = (t - s) - m
+            s = t
+        assert np.array_equal(c.cpu().numpy(), s - e), (P, opts)
+
+
 @pytest.mark.parametrize("dtype", ["f32", "f64", "bf16"])
 @pytest.mark.parametrize("nq", [34, 64, 65, 66, 71, 102, 255, 256, 257, 258, 511, 513, 514, 645, 1023, 1024, 1025, 1281, 1500,
                                 1534, 1535, 2001])

@@ -203,8 +203,7 @@ template <typename T, int N, int SUM> struct GsSum {
 #pragma unroll
         for (int u = 0; u < UB; ++u) {
             if (PART && u >= count) break;
-#pragma unroll
-            for (int n = 0; n < N; ++n) acc[n].fma_add(x[u][n], y[u][n]);
+            fma_add_all<N>(acc, x[u], y[u]);
         }
     }
     __device__ __forceinline__ void finish() {}

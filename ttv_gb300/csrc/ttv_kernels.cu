@@ -135,8 +135,10 @@ __device__ __forceinline__ void row_fma(AccT (&acc)[V], const T (&av)[V], T bb, 
                 acc[v].add_split(split_double(av[v]), bs, av[v], bb);
         }
     } else {
+        T bv[V];
 #pragma unroll
-        for (int v = 0; v < V; ++v) acc[v].fma_add(av[v], bb);
+        for (int v = 0; v < V; ++v) bv[v] = bb;
+        fma_add_all<V>(acc, av, bv);
     }
 }
 
@@ -165,8 +167,7 @@ __device__ __forceinline__ void vec_fma(AccT (&acc)[V], const T (&av)[V], const 
             }
         }
     } else {
-#pragma unroll
-        for (int v = 0; v < V; ++v) acc[v].fma_add(av[v], bv[v]);
+        fma_add_all<V>(acc, av, bv);
     }
 }
 
