@@ -154,11 +154,13 @@ __device__ __forceinline__ void kahan_pair(Acc<float, true>& p, Acc<float, true>
         : "f"(a0), "f"(a1), "f"(-b0), "f"(-b1));
 }
 
-// acc[n] += x[n] y[n]
-template <int N, typename AccT, typename T>
+// acc[n] += x[n] y[n].  PAIR off: where a sum starts in straight-line code, whose first
+// product the compiler fuses into the second step's addition (a rounding less, which
+// sums of a few terms show: 4 rows 2.9e-8, in packed steps 3.6e-8).
+template <int N, bool PAIR = true, typename AccT, typename T>
 __device__ __forceinline__ void fma_add_all(AccT (&acc)[N], const T (&x)[N], const T (&y)[N])
 {
-    if constexpr (std::is_same<AccT, Acc<float, true>>::value && N % 2 == 0) {
+    if constexpr (PAIR && std::is_same<AccT, Acc<float, true>>::value && N % 2 == 0) {
 #pragma unroll
         for (int n = 0; n < N; n += 2) kahan_pair(acc[n], acc[n + 1], x[n], x[n + 1], y[n], y[n + 1]);
     } else {

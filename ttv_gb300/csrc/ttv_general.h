@@ -34,8 +34,9 @@ struct GSArgs {
     uint32_t group_log2;          // row form: lanes per output
 };
 
-// How a thread sums: Kahan, fp64 products in fixed point, fp64 native and double-float products.
-enum GsMode { GS_KAHAN = 0, GS_FX = 1, GS_MIX = 2 };
+// How a thread sums: Kahan, fp64 products in fixed point, fp64 native and double-float products,
+// fp32 Kahan whose first product is exact.
+enum GsMode { GS_KAHAN = 0, GS_FX = 1, GS_MIX = 2, GS_FIRST = 3 };
 
 struct GSPlan {
     GSArgs k{};

@@ -112,7 +112,7 @@ template <int V> __device__ __forceinline__ constexpr bool f64_native(int u, int
 }
 
 // bsp (PRE): b's double-float split, computed once per staged segment.
-template <int V, bool PRE = false, typename AccT, typename T>
+template <int V, bool PRE = false, bool PAIR = true, typename AccT, typename T>
 __device__ __forceinline__ void row_fma(AccT (&acc)[V], const T (&av)[V], T bb, int u = 0,
                                         const float2* bsp = nullptr)
 {
@@ -138,14 +138,14 @@ __device__ __forceinline__ void row_fma(AccT (&acc)[V], const T (&av)[V], T bb, 
         T bv[V];
 #pragma unroll
         for (int v = 0; v < V; ++v) bv[v] = bb;
-        fma_add_all<V>(acc, av, bv);
+        fma_add_all<V, PAIR>(acc, av, bv);
     }
 }
 
 // acc[v] += av[v] * bv[v] (row form: b varies with the element).  The fp64
 // double-float accumulator mixes the same way: even vector slots (or even
 // unrolled loads when V == 1) on the DFMA pipe, odd ones emulated.
-template <int V, bool PRE = false, typename AccT, typename T>
+template <int V, bool PRE = false, bool PAIR = true, typename AccT, typename T>
 __device__ __forceinline__ void vec_fma(AccT (&acc)[V], const T (&av)[V], const T (&bv)[V], int u = 0,
                                         const float2* bsp = nullptr)
 {
@@ -167,7 +167,7 @@ __device__ __forceinline__ void vec_fma(AccT (&acc)[V], const T (&av)[V], const 
             }
         }
     } else {
-        fma_add_all<V>(acc, av, bv);
+        fma_add_all<V, PAIR>(acc, av, bv);
     }
 }
 
@@ -344,7 +344,7 @@ __device__ __forceinline__ void row_short(const KArgs& k, uint32_t G, uint32_t l
 #pragma unroll
             for (int v = 0; v < V; ++v) acc[v].init();
 #pragma unroll
-            for (int t = 0; t < M; ++t) vec_fma<V>(acc, av[r][t], bv[t], t);
+            for (int t = 0; t < M; ++t) vec_fma<V, false, false>(acc, av[r][t], bv[t], t);
             renorm_all<V>(acc);
             fold_vec<V>(acc);
             for (uint32_t off = G >> 1; off > 0; off >>= 1) {
@@ -498,11 +498,11 @@ __global__ void __launch_bounds__(BLOCK, (min_ctas<TA, V>())) col_short_kernel(K
                 if ((uint32_t)i < nq) {
                     if constexpr (PRES) {
                         if (split_ok)
-                            row_fma<V, true>(acc, av[h][i], bq[i], i, &bsp[i]);
+                            row_fma<V, true, false>(acc, av[h][i], bq[i], i, &bsp[i]);
                         else
-                            row_fma<V, false>(acc, av[h][i], bq[i], i, nullptr);
+                            row_fma<V, false, false>(acc, av[h][i], bq[i], i, nullptr);
                     } else {
-                        row_fma<V, false>(acc, av[h][i], bq[i], i, nullptr);
+                        row_fma<V, false, false>(acc, av[h][i], bq[i], i, nullptr);
                     }
                 }
             }
