@@ -382,7 +382,7 @@ int make_plan_inner(int dtype, const Canon& cn, const void* a, const void* b, co
 //     whole blocks of loads (2097152 x 128: 164 -> 157 us, 349525 x 192: 47.4 -> 42.0,
 //     131072 x 512: 42.2 -> 41.0; of 100, 144 and 320 level or 5 % slower);
 //   columns split by the plan: 16-byte loads up to 2^25 elements (256^3: 17.5 ->
-//     13.4 us, 2^25: 30 -> 25; 19404 x 1777 above it 29 -> 38), prefixes under 48
+//     12.2 us, 2^25: 30 -> 25; 19404 x 1777 above it 29 -> 38), prefixes under 48
 //     up to 2^21 (40 x 5242 x 20: 9.2 -> 10.8), narrower loads up to 2^23 (from
 //     2050 x 2730 x 3 on the dense kernel wins);
 //   thin prefixes with slabs of at most 2^14 elements, more of them than SMs or
@@ -390,16 +390,16 @@ int make_plan_inner(int dtype, const Canon& cn, const void* a, const void* b, co
 //     slabs are 1.4 to 4 times slower here), prefixes under 8 elements only many
 //     slabs of a small A (2 x 2138 x 16: 4.2 -> 5.7);
 //   contractions of at most 4 rows, A of 2^26 elements or more and a prefix of 16
-//     (2^28: 208 -> 197 us, 2^25: level, 2^23: 7.0 -> 8.4; a prefix of 4: 84 -> 112).
+//     (2^28: 208 -> 195 us, 2^25: level, 2^23: 7.0 -> 8.4; a prefix of 4: 84 -> 112).
 // bf16 (the dense kernels hold 32 to 64 bytes in flight per thread, these 64 and
 // more warps):
 //   rows of 96 elements or more in 16-byte loads (16384 x 4096: 38.7 -> 28.0 us,
 //     500000 x 104: 33.8 -> 30.8; 65536 x 64 level, 1000000 x 64: 40.3 -> 42.4);
 //   rows split by the plan while b stays in L1 or A is small (300000 x 101: 41.9 ->
 //     32.7, 4096 x 1001: 10.1 -> 6.2; 200 rows of 66032: 17.2 -> 19.2);
-//   thin prefixes by the fp32 rule (64^4: 17.0 -> 10.3 us);
+//   thin prefixes by the fp32 rule (64^4: 17.0 -> 9.2 us);
 //   columns in loads of two elements or more (6 x 7 x 10^6: 45.0 -> 27.8 us, 512^3:
-//     63 -> 52, 1024^2: 7.2 -> 4.3), one element up to 2^24 (1001 x 100 x 100: 13.4 ->
+//     63 -> 44, 1024^2: 7.2 -> 4.3), one element up to 2^24 (1001 x 100 x 100: 13.4 ->
 //     7.9; 301^3 25.0 -> 27.2, 501 x 7 x 10001: 37.5 -> 74.5).
 // fp64 (the dense kernels' mixed products, no second launch), without segments of
 // the grid (16 x 10000: 6.6 -> 9.2):
