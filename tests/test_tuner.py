@@ -91,6 +91,17 @@ def test_hint_that_no_longer_applies_falls_back(T):
     assert (got["kind"], got["group"], got["split"]) == (base["kind"], base["group"], base["split"])
 
 
+@pytest.mark.parametrize("na,pia,q,dtype", [([256, 256, 256], [1, 2, 3], 2, "F32"), ([512, 512, 512], [1, 2, 3], 2, "BF16A"),
+                                            ([64, 64, 64], [1, 2, 3], 2, "F64"), ([128, 1 << 16], [1, 2], 1, "F32"),
+                                            ([645, 645, 645], [1, 2, 3], 2, "F32")])
+def test_hint_of_the_planners_own_choice_changes_nothing(T, na, pia, q, dtype):
+    # the tuner's first candidate is {}: where it wins, installing it must leave the plan it timed
+    dt = getattr(T, dtype)
+    base = T.plan(q, na, pia, dtype=dt)
+    TU.install([{"dtype": dt, "P": base["P"], "nq": base["nq"], "S": base["S"], "options": {}}])
+    assert T.plan(q, na, pia, dtype=dt) == base
+
+
 def test_clear_all_hints(T):
     for P in (16, 32, 64):
         T.plan_hint(T.F32, P, 4096, 1, kind=T.KIND_COL, split=7)

@@ -477,7 +477,9 @@ int make_plan(int dtype, const Canon& cn, const void* a, const void* b, const tl
         {
             std::lock_guard<std::mutex> lk(g_hint_mu);
             auto it = g_hints.find(std::make_tuple(dtype, cn.P, cn.nq, cn.S));
-            if (it != g_hints.end()) {
+            // (a hint that leaves every choice open, as the tuner stores where the planner's own
+            // choice won, is that choice: the rules below, general-stride kernels included)
+            if (it != g_hints.end() && !default_choices(&it->second)) {
                 hinted = it->second;
                 found = true;
             }
