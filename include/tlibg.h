@@ -168,7 +168,9 @@ int tlibg_ttvs_packed_rowmajor(const uint64_t* words);
  * vector is taken, as long as no two outputs share an element of C
  * (TLIBG_ERR_UNSUPPORTED otherwise) and every offset stays below 2^62.
  * dtype TLIBG_F32 or TLIBG_F64; compensated accumulation; asynchronous on
- * `stream`.  Views that are dense take the dense kernels' speed only through
+ * `stream`.  Views of few outputs over a long contraction use the stream's
+ * cached scratch (allocated on the first such call); calls on a stream under
+ * capture use none.  Views that are dense take the dense kernels' speed only through
  * tlibg_ttv_*. */
 int tlibg_ttv_strided(int dtype, size_t q, size_t p,
                       const void* a, const size_t* na, const size_t* wa, const size_t* pia,

@@ -249,3 +249,107 @@ def test_fp64_nonfinite_products(engine, cuda):
         bad = torch.zeros(37, dtype=torch.bool, device=cuda)
         bad[[3, 8, 20]] = True
         assert not torch.isfinite(c[bad]).any() and torch.isfinite(c[~bad]).all()
+
+
+def _captured(torch, fn, stream):
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=stream):
+        fn()
+    return graph
+
+
+@pytest.mark.parametrize("shape,q", [((2, 700001), 2), ((900001, 3), 1)], ids=["rows", "columns"])
+def test_captured_views_need_no_scratch(engine, cuda, shape, q):
+    """A view of few outputs, whose eager call allocates scratch for segments of the contraction,
+    is captured on a stream that never had any, and replayed on new data after a larger eager call."""
+    import torch
+    g = torch.Generator(device=cuda)
+    g.manual_seed(5)
+    base = torch.empty(shape[0], shape[1] + 1, device=cuda)
+    A, b = base[:, :shape[1]], torch.empty(shape[q - 1], device=cuda)
+    c = torch.empty(shape[2 - q], device=cuda)
+
+    def check():
+        ref, absn = torch.mv(A.double() if q == 2 else A.double().T, b.double()), A.double().abs().sum(q - 1)
+        assert ((c.double() - ref).abs() <= 4 * 2.0 ** -24 * absn).all()
+
+    def fill():
+        base.uniform_(-1, 1, generator=g)
+        b.uniform_(-1, 1, generator=g)
+        c.fill_(float("nan"))
+
+    fill()
+    fresh, s = torch.cuda.Stream(), torch.cuda.Stream()
+    before = engine.device_alloc_count()
+    engine.ttv_view(q, A, b, out=c, stream=fresh)
+    torch.cuda.synchronize()
+    assert engine.device_alloc_count() == before + 1
+    check()
+    graph = _captured(torch, lambda: engine.ttv_view(q, A, b, out=c, stream=s), s)
+    assert engine.device_alloc_count() == before + 1
+    for _ in range(2):
+        fill()
+        graph.replay()
+        torch.cuda.synchronize()
+        check()
+        wide = torch.rand(4, 1 << 20, device=cuda)[:, 1:]
+        engine.ttv_view(2, wide, wide[0], stream=s)
+        torch.cuda.synchronize()
+
+
+def test_captured_scratch_outlives_its_growth(engine, cuda):
+    """A captured split call keeps its scratch when a later call on the stream outgrows it; a split
+    plan captured on a stream without scratch runs unsplit."""
+    import torch
+    g = torch.Generator(device=cuda)
+    g.manual_seed(6)
+
+    def problem(P, nq, S, **opts):
+        a, b = torch.empty(S, nq, P, device=cuda), torch.empty(nq, device=cuda)
+        c = torch.empty(S, P, device=cuda)
+
+        def call():
+            engine.ttv(2, 3, a, [P, nq, S], [1, P, P * nq], [1, 2, 3], b, [nq], c, [P, S], [1, P], [1, 2], **opts)
+
+        def fill():
+            for t in (a, b):
+                t.uniform_(-1, 1, generator=g)
+            c.fill_(float("nan"))
+
+        def check():
+            ref = torch.einsum("sip,i->sp", a.double(), b.double())
+            absn = torch.einsum("sip,i->sp", a.double().abs(), b.double().abs())
+            assert ((c.double() - ref).abs() <= 4 * 2.0 ** -24 * absn).all()
+        return call, fill, check
+
+    s = torch.cuda.Stream()
+    small, fill, check = problem(1024, 512, 1, kind=engine.KIND_COL, split=8)
+    large, fill2, check2 = problem(16384, 512, 1, kind=engine.KIND_COL, split=32)
+    fill()
+    fill2()
+    torch.cuda.synchronize()
+    with torch.cuda.stream(s):
+        small()
+    graph = _captured(torch, small, s)
+    before = engine.device_alloc_count()
+    with torch.cuda.stream(s):
+        large()
+    torch.cuda.synchronize()
+    assert engine.device_alloc_count() == before + 1
+    check2()
+    for _ in range(2):
+        fill()
+        torch.cuda.synchronize()
+        graph.replay()
+        with torch.cuda.stream(s):
+            large()
+        torch.cuda.synchronize()
+        check()
+    planned, fill, check = problem(4, 128, 20000)
+    assert engine.plan(2, [4, 128, 20000], [1, 2, 3])["split"] > 1
+    graph = _captured(torch, planned, torch.cuda.Stream())
+    fill()
+    graph.replay()
+    torch.cuda.synchronize()
+    check()
+    assert engine.device_error() == 0

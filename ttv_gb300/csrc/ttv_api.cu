@@ -999,12 +999,36 @@ int make_plan_inner(int dtype, const Canon& cn, const void* a, const void* b, co
 // --------------------------------------------------------------------------
 // per-(device, stream) scratch for split partials (grow-only)
 // --------------------------------------------------------------------------
+// A buffer handed out while its stream is being captured stays in the graph, so an
+// outgrown one is then kept instead of freed; the next is at least twice its size, so
+// the kept ones together stay below the one in use.
 struct Scratch {
     void* ptr = nullptr;
     size_t bytes = 0;
+    bool captured = false;
 };
 std::mutex g_scratch_mu;
 std::map<std::pair<int, uintptr_t>, Scratch> g_scratch;
+
+bool capturing(cudaStream_t stream)
+{
+    cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(stream, &status) != cudaSuccess) {
+        cudaGetLastError();   // the legacy stream while another stream is being captured
+        return false;
+    }
+    return status == cudaStreamCaptureStatusActive;
+}
+
+// Whether the stream's scratch holds `bytes` already.
+bool scratch_ready(cudaStream_t stream, size_t bytes)
+{
+    int dev = 0;
+    cudaGetDevice(&dev);
+    std::lock_guard<std::mutex> lk(g_scratch_mu);
+    auto it = g_scratch.find({dev, reinterpret_cast<uintptr_t>(stream)});
+    return it != g_scratch.end() && it->second.bytes >= bytes;
+}
 
 int get_scratch(cudaStream_t stream, size_t bytes, void** out)
 {
@@ -1014,24 +1038,30 @@ int get_scratch(cudaStream_t stream, size_t bytes, void** out)
     }
     int dev = 0;
     cudaGetDevice(&dev);
+    const bool in_graph = capturing(stream);
     std::lock_guard<std::mutex> lk(g_scratch_mu);
     Scratch& s = g_scratch[{dev, reinterpret_cast<uintptr_t>(stream)}];
     if (s.bytes < bytes) {
-        if (s.ptr) {
+        const bool keep = s.captured || in_graph;
+        const size_t want = std::max({bytes, (size_t)1 << 20, keep ? 2 * s.bytes : 0});
+        if (s.ptr && !keep) {
             // the previous buffer may still be read by work queued on this stream
             cudaStreamSynchronize(stream);
             cudaFree(s.ptr);
             s.ptr = nullptr;
             s.bytes = 0;
         }
-        size_t want = std::max(bytes, (size_t)1 << 20);
-        cudaError_t e = device_malloc(&s.ptr, want);
+        void* grown = nullptr;
+        cudaError_t e = device_malloc(&grown, want);
         if (e != cudaSuccess) {
             cudaGetLastError();
             return fail(TLIBG_ERR_NOMEM, std::string("tlibg: cannot allocate split scratch: ") + cudaGetErrorString(e));
         }
+        s.ptr = grown;
         s.bytes = want;
+        s.captured = false;
     }
+    s.captured = s.captured || in_graph;
     *out = s.ptr;
     return TLIBG_OK;
 }
@@ -1114,6 +1144,13 @@ int run_device(int dtype, size_t q, size_t p, const void* a, const size_t* na, c
     Plan pl;
     st = make_plan(dtype, cn, a, b, opt, d.sms, &pl);
     if (st) return st;
+    // a captured call whose scratch was never allocated runs unsplit: allocating would
+    // end the capture
+    if (default_choices(opt) && partial_bytes(pl) && capturing(stream) && !scratch_ready(stream, partial_bytes(pl))) {
+        const tlibg_options whole{TLIBG_ACC_COMPENSATED, -1, 0, 0, 1, 0};
+        Plan alt;
+        if (make_plan_inner(dtype, cn, a, b, &whole, d.sms, &alt) == TLIBG_OK && partial_bytes(alt) == 0) pl = alt;
+    }
     void* part = nullptr;
     st = get_scratch(stream, partial_bytes(pl), &part);
     if (st) return st;
@@ -1356,6 +1393,10 @@ int tlibg_ttv_strided(int dtype, size_t q, size_t p, const void* a, const size_t
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     pl.dtype = dtype;
     gs_plan(sms, &pl);
+    // Captured calls share the contraction over a cluster at most: a graph that held the
+    // stream's scratch could not be replayed beside the stream's other calls, and could
+    // not be captured before the scratch is there
+    if (pl.k.nseg > 1 && capturing(st)) gs_plan(sms, &pl, false);
     if (pl.k.nseg > 1)
         if (int s = get_scratch(st, gs_partial_bytes(pl), &pl.k.part)) return s;
     uint64_t launches = 0;

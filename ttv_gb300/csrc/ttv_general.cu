@@ -824,7 +824,7 @@ static int gs_ctas_per_sm(const GSPlan& p, bool share)
 // (clocks swept from 1200 to 2000, the cost of sharing from 600 to 5500).
 // `rows`: loads along q of an unsplit warp (row form: of a lane); N: elements a
 // lane loads per row.
-static void gs_split(GSPlan* p, uint64_t rows, bool may_split, uint32_t outs_per_warp, int N, int sms)
+static void gs_split(GSPlan* p, uint64_t rows, bool may_split, bool segments, uint32_t outs_per_warp, int N, int sms)
 {
     GSArgs& k = p->k;
     int U = 1;
@@ -844,7 +844,7 @@ static void gs_split(GSPlan* p, uint64_t rows, bool may_split, uint32_t outs_per
             const int cps = cps_of[wl > 0];
             const uint64_t ctas = tiles(wl) << cl, cap = (uint64_t)sms * cps;
             uint64_t ns = 1;
-            if (wl == 3 && cl == 3 && ctas < cap) ns = std::max<uint64_t>(1, std::min<uint64_t>(cap / ctas, rows / (64 * 16)));
+            if (segments && wl == 3 && cl == 3 && ctas < cap) ns = std::max<uint64_t>(1, std::min<uint64_t>(cap / ctas, rows / (64 * 16)));
             const uint64_t ways = (uint64_t)(1u << (wl + cl)) * ns;
             if (ways > 1 && (!may_split || rows < 2 * ways)) continue;
             const double fixed = 1500 + (wl ? (p->mix ? 3000 : 5000) : 0) + (cl ? (p->mix ? 5000 : 6000) : 0) + (ns > 1 ? 6000 : 0);
@@ -874,7 +874,7 @@ static void gs_split(GSPlan* p, uint64_t rows, bool may_split, uint32_t outs_per
     p->grid = (int)(std::min<uint64_t>(k.items, ((uint64_t)sms * 32) >> k.cluster_log2) << k.cluster_log2);
 }
 
-void gs_plan(int sms, GSPlan* p)
+void gs_plan(int sms, GSPlan* p, bool segments)
 {
     GSArgs& k = p->k;
     const bool f64 = p->dtype == F64, bf16 = p->dtype == BF16A;
@@ -911,7 +911,7 @@ void gs_plan(int sms, GSPlan* p)
         // (16-byte fp32 vectors: two at most, four spill; bf16 ones hold eight sums already)
         p->M = plain || p->mix || lane_rows > 4 || p->V == 8 ? 1 : (lane_rows > 2 || p->V == 4 ? 2 : 4);
         while (p->M > 1 && (k.outputs << gl) < lanes * p->M) p->M /= 2;
-        gs_split(p, lane_rows, gl == 5, (uint32_t)((32u >> gl) * p->M), p->V * p->M, sms);
+        gs_split(p, lane_rows, gl == 5, segments, (uint32_t)((32u >> gl) * p->M), p->V * p->M, sms);
     } else {
         auto columns = [&](uint64_t v) { return k.wa[0] == 1 && k.ext[0].d % v == 0 && k.waq % v == 0 && on_grid(v); };
         p->V = !plain && columns(V) ? (int)V : 1;
@@ -927,7 +927,7 @@ void gs_plan(int sms, GSPlan* p)
         } else {        // two in long ones, one where there are too few to fill the chip
             p->M = !f64 && k.nq >= 64 && k.outputs >= lanes ? 2 : 1;
         }
-        gs_split(p, k.nq, true, (uint32_t)(32 * p->V * p->M), p->V * p->M, sms);
+        gs_split(p, k.nq, true, segments, (uint32_t)(32 * p->V * p->M), p->V * p->M, sms);
     }
 }
 

@@ -51,8 +51,9 @@ struct GSPlan {
 // The modes other than q as (A stride, extent, C stride); extents of 1 left out.
 void gs_modes(std::vector<std::tuple<size_t, size_t, size_t>> modes, GSArgs* k);
 
-// Form, vector width and split for the args' modes, a, b, nq, waq and wb.
-void gs_plan(int sms, GSPlan* p);
+// Form, vector width and split for the args' modes, a, b, nq, waq and wb; without
+// `segments` the split stays within a cluster and needs no scratch.
+void gs_plan(int sms, GSPlan* p, bool segments = true);
 
 // Enqueues a plan's kernels; `dependent`: as a programmatic dependent of the
 // stream's previous kernel.
