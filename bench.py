@@ -203,7 +203,9 @@ def kernel_label(T, c):
            T.KIND_COL_THIN: "col_thin_kernel", T.KIND_ROW_TILE: "row_tile_kernel",
            T.KIND_COL_BULK: "col_bulk_kernel", T.KIND_ROW_PANEL: "row_panel_kernel",
            T.KIND_ROW_SHIFT: "row_shift_kernel"}[pl["kind"]]
-    if pl["kind"] == T.KIND_COL and pl["vec"] == 1:
+    if pl["cluster"]:
+        fam = "gs_row_kernel" if pl["kind"] == T.KIND_ROW else "gs_col_kernel"
+    elif pl["kind"] == T.KIND_COL and pl["vec"] == 1:
         fam = "col_strided_kernel"   # scalar loads, two outputs per thread
     templ = "" if pl["kind"] in (T.KIND_STREAM, T.KIND_ROW_TILE, T.KIND_COL_BULK) else f",V{pl['vec']}"
     if pl["kind"] == T.KIND_ROW_PANEL:

@@ -86,11 +86,16 @@ typedef struct tlibg_options {
     int sync;         /* nonzero: synchronise `stream` and check the device error word    */
 } tlibg_options;
 
-/* Launch configuration the planner picks for a canonical problem. */
+/* Launch configuration the planner picks for a canonical problem.  `cluster` tells
+ * the two implementations of TLIBG_KIND_ROW and TLIBG_KIND_COL apart: 0, the dense
+ * kernels, which kind, group, vec and split given as options run again; from 1 on,
+ * the general-stride kernels with clusters of that many CTAs, which the planner alone
+ * chooses (the same values as options select a dense kernel). */
 typedef struct tlibg_plan_info {
     uint64_t P, nq, S;   /* prefix before q in the layout, contracted extent, suffix      */
     int kind, group, vec, split, accumulate;
     int grid, block;
+    int cluster;
 } tlibg_plan_info;
 
 /* ---------------------------------------------------------------------------

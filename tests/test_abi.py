@@ -567,3 +567,19 @@ def test_python_calls_keep_their_answers(engine):
         engine.ttv(1, 3, t, *meta, b, [4], c, *out, no_such_option=1)
     with pytest.raises(engine.TTVError, match="contraction dimension of A and B are not equal"):
         engine.ttv_array(2, torch.zeros(4, 5), torch.zeros(4))
+
+
+def _general(engine, dtype, P, nq, S):
+    pl = engine.plan(2, [P, nq, S], [1, 2, 3], dtype=dtype)
+    return pl["kind"], pl["cluster"] > 0
+
+
+def test_plan_tells_the_two_column_kernels_apart(engine):
+    """plan() names the kernels that run: general-stride plans carry their cluster size, and their
+    kind, group, vec and split as options are a dense plan's."""
+    pl = engine.plan(2, [256, 256, 256], [1, 2, 3])
+    assert pl["kind"] == engine.KIND_COL and pl["cluster"] >= 1
+    back = engine.plan(2, [256, 256, 256], [1, 2, 3], kind=pl["kind"], group=pl["group"], vec=pl["vec"], split=pl["split"])
+    assert back["cluster"] == 0
+    assert engine.plan(2, [645, 645, 645], [1, 2, 3])["cluster"] == 0
+    assert engine.plan(1, [64, 12], [1, 2], kind=engine.KIND_ROW)["cluster"] == 0

@@ -65,7 +65,7 @@ class Options(C.Structure):
 class PlanInfo(C.Structure):
     _fields_ = [("P", C.c_uint64), ("nq", C.c_uint64), ("S", C.c_uint64), ("kind", C.c_int),
                 ("group", C.c_int), ("vec", C.c_int), ("split", C.c_int),
-                ("accumulate", C.c_int), ("grid", C.c_int), ("block", C.c_int)]
+                ("accumulate", C.c_int), ("grid", C.c_int), ("block", C.c_int), ("cluster", C.c_int)]
 
     def as_dict(self):
         return {f: getattr(self, f) for f, _ in self._fields_}

@@ -1322,6 +1322,7 @@ int tlibg_plan(int dtype, size_t q, size_t p, const size_t* na, const size_t* pi
     out->split = pl.split;
     out->accumulate = pl.kahan ? TLIBG_ACC_COMPENSATED : TLIBG_ACC_PLAIN;
     out->grid = pl.grid;
+    out->cluster = pl.general ? 1 << pl.gs.k.cluster_log2 : 0;
     out->block = pl.kind == KIND_STREAM ? STREAM_CONSUMERS + 32
                  : (pl.kind == KIND_ROW_TILE ? ROWT_THREADS : (pl.kind == KIND_COL_BULK ? CB_THREADS : BLOCK));
     return ok();
