@@ -583,3 +583,12 @@ def test_plan_tells_the_two_column_kernels_apart(engine):
     assert back["cluster"] == 0
     assert engine.plan(2, [645, 645, 645], [1, 2, 3])["cluster"] == 0
     assert engine.plan(1, [64, 12], [1, 2], kind=engine.KIND_ROW)["cluster"] == 0
+
+
+def test_unsplit_rows_leave_the_dense_kernel_only_in_whole_blocks(engine):
+    """fp32 rows of a multiple of 64 elements run on the general-stride kernel where every lane's
+    loads are whole blocks of four, and on the dense kernel, faster there, where they are not."""
+    for nq in (128, 192, 384, 512, 1536, 2048):
+        assert _general(engine, engine.F32, 1, nq, (1 << 27) // nq) == (engine.KIND_ROW, True), nq
+    for nq in (320, 448, 576, 640, 704, 960, 1088, 1344, 1920):
+        assert _general(engine, engine.F32, 1, nq, (1 << 27) // nq) == (engine.KIND_ROW, False), nq

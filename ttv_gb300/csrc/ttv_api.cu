@@ -379,8 +379,9 @@ int make_plan_inner(int dtype, const Canon& cn, const void* a, const void* b, co
 //     2^24 (512 x 4096: 6.9 -> 2.9 us, 4096 x 4096: 15.9 -> 11.4), level at 2^26
 //     (rows over 2^16 long slower there: 256 x 262144: 45.8 -> 47.4);
 //   unsplit rows of a multiple of 64 elements in 16-byte loads, whose lanes all take
-//     whole blocks of loads (2097152 x 128: 164 -> 157 us, 349525 x 192: 47.4 -> 42.0,
-//     131072 x 512: 42.2 -> 41.0; of 100, 144 and 320 level or 5 % slower);
+//     whole blocks of four loads (2097152 x 128: 164 -> 157 us, 349525 x 192: 47.4 -> 42.0,
+//     131072 x 512: 42.2 -> 41.0; others end in masked blocks: 104857 x 320 23.1 -> 24.3,
+//     58254 x 576 22.3 -> 25.2, 24966 x 1344 23.0 -> 27.1, of 100 and 144 level or 5 % slower);
 //   columns split by the plan: 16-byte loads up to 2^25 elements (256^3: 17.5 ->
 //     12.2 us, 2^25: 30 -> 25; 19404 x 1777 above it 29 -> 38), prefixes under 48
 //     up to 2^21 (40 x 5242 x 20: 9.2 -> 10.8), narrower loads up to 2^23 (from
@@ -451,6 +452,10 @@ void route_general(const Canon& cn, const void* a, const void* b, int sms, Plan*
     g.k.waq = cn.nq > 1 ? cn.P : 0;
     g.k.wb = 1;
     gs_plan(sms, &g);
+    if (pl->kind == KIND_ROW && !f64 && !bf16 && pl->split == 1) {
+        const uint64_t loads = cn.nq / g.V;   // whole blocks of four for every lane
+        if (loads % (uint64_t(4) << g.k.group_log2) != 0) return;
+    }
     if (f64) {
         if (g.k.nseg > 1) return;
         const uint64_t most = g.V == 2 ? (g.k.wi_log2 || cn.nq <= 8 ? 26 : 23) : (cn.nq >= 64 ? 24 : 22);
