@@ -592,3 +592,14 @@ def test_unsplit_rows_leave_the_dense_kernel_only_in_whole_blocks(engine):
         assert _general(engine, engine.F32, 1, nq, (1 << 27) // nq) == (engine.KIND_ROW, True), nq
     for nq in (320, 448, 576, 640, 704, 960, 1088, 1344, 1920):
         assert _general(engine, engine.F32, 1, nq, (1 << 27) // nq) == (engine.KIND_ROW, False), nq
+
+
+def test_short_contractions_stay_on_the_dense_kernels(engine):
+    """A few rows of large column problems: bf16 storage up to 6 rows (over 2 of them only below
+    2^26 elements), fp64 up to 8 from 2^22 elements on."""
+    for P, nq, S, general in ((32768, 1, 4096, False), (32768, 2, 1024, False), (4096, 4, 2048, False), (4096, 6, 1365, False),
+                              (4096, 4, 1 << 15, True), (4096, 8, 2048, True), (4096, 12, 1365, True)):
+        assert _general(engine, engine.BF16A, P, nq, S) == (engine.KIND_COL, general), (P, nq, S)
+    for P, nq, S, general in ((32768, 1, 512, False), (32768, 3, 170, False), (512, 8, 4096, False), (4096, 5, 819, False),
+                              (32768, 3, 10, True), (32768, 4, 8, True)):
+        assert _general(engine, engine.F64, P, nq, S) == (engine.KIND_COL, general), (P, nq, S)

@@ -400,15 +400,21 @@ int make_plan_inner(int dtype, const Canon& cn, const void* a, const void* b, co
 //     32.7, 4096 x 1001: 10.1 -> 6.2; 200 rows of 66032: 17.2 -> 19.2);
 //   thin prefixes by the fp32 rule (64^4: 17.0 -> 9.2 us);
 //   columns in loads of two elements or more (6 x 7 x 10^6: 45.0 -> 27.8 us, 512^3:
-//     63 -> 44, 1024^2: 7.2 -> 4.3), one element up to 2^24 (1001 x 100 x 100: 13.4 ->
-//     7.9; 301^3 25.0 -> 27.2, 501 x 7 x 10001: 37.5 -> 74.5).
+//     63 -> 44, 1024^2: 7.2 -> 4.3), but not of up to six rows in 16-byte loads whose tiles
+//     fill the GPU unsplit, over two of them below 2^26 elements (2^27 elements of 1 row
+//     206 -> 293 us, 2 rows 114 -> 131, 4 rows 76 -> 74; 2^25: 4 rows 23.1 -> 31.2, 6 rows
+//     21.1 -> 23.0, 8 rows 19.2 -> 18.0; 2^20, whose tiles do not: 1 row 7.7 -> 6.6);
+//     one element up to 2^24 (1001 x 100 x 100: 13.4 -> 7.9; 301^3 25.0 -> 27.2, 501 x 7 x
+//     10001: 37.5 -> 74.5).
 // fp64 (the dense kernels' mixed products, no second launch), without segments of
 // the grid (16 x 10000: 6.6 -> 9.2):
 //   rows that the plan splits, up to 3 x 2^22 elements (1024 x 4096: 18.3 -> 10.6 us,
 //     4000 x 2001: 23.2 -> 17.1; 4096 x 4096: 30.5 -> 35.2), others up to 2^21;
-//   columns in 16-byte loads up to 2^26 elements where warps share the contraction or
-//     it is at most 8 long (256^3: 33.3 -> 27.9, 128^3: 8.3 -> 6.0, 1024^2: 7.4 -> 5.3;
-//     512^3: 168.6 -> 171.9), else 2^23 (8 x 16 x 100000: 22.0 -> 22.3);
+//   columns in 16-byte loads up to 2^26 elements where warps share the contraction
+//     (256^3: 33.3 -> 27.9, 128^3: 8.3 -> 6.0, 1024^2: 7.4 -> 5.3; 512^3: 168.6 -> 171.9),
+//     else 2^23 (8 x 16 x 100000: 22.0 -> 22.3), at most 8 rows that the dense kernels
+//     neither split nor share 2^22, three rows 2^21 (2^20 elements of 3 rows 5.3 -> 4.8 us,
+//     2^22: 13.4 -> 14.9, 2^24: 41 -> 50, 5 rows 35.8 -> 38.0, 8 rows 29.3 -> 31.5);
 //   columns in single loads up to 2^24 elements, of under 64 rows 2^22 (31 x 100 x
 //     3000: 26.2 -> 18.7; 645 x 645 x 64: 51 -> 59, 301 x 7 x 3000: 18.0 -> 22.6).
 // Contractions over more than 2^20 elements keep the dense kernels' combine.
@@ -429,12 +435,16 @@ void route_general(const Canon& cn, const void* a, const void* b, int sms, Plan*
                                  : pl->vec == 4 && cn.nq % 64 == 0;
         }
     } else if (f64) {   // and, below, by the plan's vectors and sharing
-        take = (pl->kind == KIND_COL_THIN || pl->kind == KIND_COL) && elems <= (uint64_t(1) << 26);
+        if (pl->kind == KIND_COL_THIN) take = true;
+        else if (pl->kind == KIND_COL) take = !(pl->rows_m == 1 || (cn.nq <= 8 && pl->group == 1 && pl->split == 1)) || elems <= (uint64_t(1) << (cn.nq >= 4 ? 22 : 21));
+        take = take && elems <= (uint64_t(1) << 26);
     } else if (pl->kind == KIND_COL_THIN) {
         take = cn.nq * cn.P <= (uint64_t(1) << 14) &&
                (cn.P >= 8 ? cn.S > (uint64_t)sms || pl->split > 1 : cn.S > (uint64_t)sms && elems <= (uint64_t(1) << 18));
     } else if (pl->kind == KIND_COL) {
-        if (bf16) take = pl->vec >= 2 || elems <= (uint64_t(1) << 24);
+        if (bf16 && pl->vec == 8 && pl->group == 1 && pl->split == 1 && cn.nq <= 6)
+            take = cn.nq > 2 && elems >= (uint64_t(1) << 26);
+        else if (bf16) take = pl->vec >= 2 || elems <= (uint64_t(1) << 24);
         else if (pl->rows_m == 1) take = elems >= (uint64_t(1) << 26) && cn.P >= 16;
         else take = pl->split > 1 && elems <= (uint64_t(1) << (pl->vec < 4 ? 23 : (cn.P >= 48 ? 25 : 21)));
     }
