@@ -603,3 +603,16 @@ def test_short_contractions_stay_on_the_dense_kernels(engine):
     for P, nq, S, general in ((32768, 1, 512, False), (32768, 3, 170, False), (512, 8, 4096, False), (4096, 5, 819, False),
                               (32768, 3, 10, True), (32768, 4, 8, True)):
         assert _general(engine, engine.F64, P, nq, S) == (engine.KIND_COL, general), (P, nq, S)
+
+
+def test_thin_prefixes_stay_on_their_kernel_in_one_wave(engine):
+    """Slabs that all have a resident CTA, and a few split ones of narrow prefixes: the thin kernel;
+    a few rows, long slabs and many slabs: the general-stride kernels."""
+    thin, gs = (engine.KIND_COL_THIN, False), (engine.KIND_COL, True)
+    for dt, P, nq, S, want in ((engine.F32, 2, 256, 200, thin), (engine.F32, 8, 512, 256, thin), (engine.F32, 16, 64, 200, thin),
+                               (engine.F32, 8, 1900, 4, thin), (engine.F32, 64, 4, 200, gs), (engine.F32, 8, 9, 400, gs),
+                               (engine.F32, 64, 200, 12, gs), (engine.F32, 16, 5, 3000, gs),
+                               (engine.BF16A, 2, 64, 256, thin), (engine.BF16A, 8, 100, 200, thin), (engine.BF16A, 2, 256, 1500, thin),
+                               (engine.BF16A, 8, 9, 200, gs), (engine.BF16A, 2, 32, 8000, gs),
+                               (engine.F64, 2, 256, 200, thin), (engine.F64, 8, 200, 2, thin), (engine.F64, 8, 700, 2, gs)):
+        assert _general(engine, dt, P, nq, S) == want, (dt, P, nq, S)

@@ -386,10 +386,15 @@ int make_plan_inner(int dtype, const Canon& cn, const void* a, const void* b, co
 //     12.2 us, 2^25: 30 -> 25; 19404 x 1777 above it 29 -> 38), prefixes under 48
 //     up to 2^21 (40 x 5242 x 20: 9.2 -> 10.8), narrower loads up to 2^23 (from
 //     2050 x 2730 x 3 on the dense kernel wins);
-//   thin prefixes with slabs of at most 2^14 elements, more of them than SMs or
-//     split by the plan (64 x 4 x 4096: 9.9 -> 2.3 us, 128^3: 5.5 -> 4.1; longer
-//     slabs are 1.4 to 4 times slower here), prefixes under 8 elements only many
-//     slabs of a small A (2 x 2138 x 16: 4.2 -> 5.7);
+//   thin prefixes with slabs of at most 2^14 elements (64 x 4 x 4096: 9.9 -> 2.3 us,
+//     128^3: 5.5 -> 4.1; longer slabs are 1.4 to 4 times slower here): more of them
+//     than fit the GPU as CTAs of the thin kernel, four per SM (then slabs of 2^13 and
+//     more only up to 2^24 elements: 4096 of 64 x 128 24.5 -> 25.8), or the plan splits
+//     them (prefixes of 16 and more: 8 x 1900 4.0 -> 4.5); between, where each slab has
+//     its CTA, slabs of 2^13 and more (200 of 64 x 128: 4.8 -> 3.7) and, from two per SM,
+//     of up to 64 rows and 2^11 elements (400 of 16 x 20 3.3 -> 2.8, but 256 of 2 x 256 2.9 ->
+//     5.0, 256 of 8 x 512 3.4 -> 4.6); prefixes under 8 elements only many slabs of a small A
+//     (2 x 2138 x 16: 4.2 -> 5.7); slabs too short for the thin kernel's warps always;
 //   contractions of at most 4 rows, A of 2^26 elements or more and a prefix of 16
 //     (2^28: 208 -> 195 us, 2^25: level, 2^23: 7.0 -> 8.4; a prefix of 4: 84 -> 112).
 // bf16 (the dense kernels hold 32 to 64 bytes in flight per thread, these 64 and
@@ -398,7 +403,9 @@ int make_plan_inner(int dtype, const Canon& cn, const void* a, const void* b, co
 //     500000 x 104: 33.8 -> 30.8; 65536 x 64 level, 1000000 x 64: 40.3 -> 42.4);
 //   rows split by the plan while b stays in L1 or A is small (300000 x 101: 41.9 ->
 //     32.7, 4096 x 1001: 10.1 -> 6.2; 200 rows of 66032: 17.2 -> 19.2);
-//   thin prefixes by the fp32 rule (64^4: 17.0 -> 9.2 us);
+//   thin prefixes of 8 and more (64^4: 17.0 -> 9.2 us), of under 100 rows where each slab
+//     has its CTA (256 of 8 x 256: 4.2 -> 5.2), narrower ones from 16 SMs' worth of outputs
+//     on (256 of 2 x 64: 2.8 -> 4.8 us);
 //   columns in loads of two elements or more (6 x 7 x 10^6: 45.0 -> 27.8 us, 512^3:
 //     63 -> 44, 1024^2: 7.2 -> 4.3), but not of up to six rows in 16-byte loads whose tiles
 //     fill the GPU unsplit, over two of them below 2^26 elements (2^27 elements of 1 row
@@ -408,6 +415,9 @@ int make_plan_inner(int dtype, const Canon& cn, const void* a, const void* b, co
 //     10001: 37.5 -> 74.5).
 // fp64 (the dense kernels' mixed products, no second launch), without segments of
 // the grid (16 x 10000: 6.6 -> 9.2):
+//   thin prefixes, but not a narrow one of over 128 rows while each slab has its CTA (256 of
+//     2 x 256: 5.1 -> 6.4 us), nor few slabs of over 100 rows that the plan does not split (40 of
+//     8 x 200: 3.9 -> 4.9) or 8 wide of over 1024 (12 of 8 x 1900: 5.6 -> 6.5; 12 x 700 5.5 -> 4.6);
 //   rows that the plan splits, up to 3 x 2^22 elements (1024 x 4096: 18.3 -> 10.6 us,
 //     4000 x 2001: 23.2 -> 17.1; 4096 x 4096: 30.5 -> 35.2), others up to 2^21;
 //   columns in 16-byte loads up to 2^26 elements where warps share the contraction
@@ -435,14 +445,22 @@ void route_general(const Canon& cn, const void* a, const void* b, int sms, Plan*
                                  : pl->vec == 4 && cn.nq % 64 == 0;
         }
     } else if (f64) {   // and, below, by the plan's vectors and sharing
-        if (pl->kind == KIND_COL_THIN) take = true;
+        if (pl->kind == KIND_COL_THIN && cn.P >= 8 && cn.S <= (uint64_t)sms) take = cn.nq <= 100 || (pl->split > 1 && (cn.P > 8 || cn.nq <= 1024 || cn.S >= 64));
+        else if (pl->kind == KIND_COL_THIN) take = cn.P >= 8 || cn.nq <= 128 || cn.S > 4 * (uint64_t)sms;
         else if (pl->kind == KIND_COL) take = !(pl->rows_m == 1 || (cn.nq <= 8 && pl->group == 1 && pl->split == 1)) || elems <= (uint64_t(1) << (cn.nq >= 4 ? 22 : 21));
         take = take && elems <= (uint64_t(1) << 26);
     } else if (pl->kind == KIND_COL_THIN) {
-        take = cn.nq * cn.P <= (uint64_t(1) << 14) &&
-               (cn.P >= 8 ? cn.S > (uint64_t)sms || pl->split > 1 : cn.S > (uint64_t)sms && elems <= (uint64_t(1) << 18));
+        const uint64_t slab = cn.nq * cn.P;
+        const bool wave = cn.S <= 4 * (uint64_t)sms;   // the thin kernel's CTAs, a slab each, all resident
+        if (cn.S <= (uint64_t)sms) take = cn.P >= 16 && pl->split > 1;
+        else if (cn.P < 8) take = elems <= (uint64_t(1) << 18) && (bf16 ? cn.P * cn.S >= 16 * (uint64_t)sms : !wave);
+        else if (bf16) take = !wave || cn.nq < 100;
+        else if (wave) take = slab >= (uint64_t(1) << 13) || (cn.S >= 2 * (uint64_t)sms && cn.nq <= 64 && slab <= (uint64_t(1) << 11));
+        else take = slab < (uint64_t(1) << 13) || elems <= (uint64_t(1) << 24);
+        take = take && slab <= (uint64_t(1) << 14);
     } else if (pl->kind == KIND_COL) {
-        if (bf16 && pl->vec == 8 && pl->group == 1 && pl->split == 1 && cn.nq <= 6)
+        if (pl->small_slabs && !bf16) take = true;
+        else if (bf16 && pl->vec == 8 && pl->group == 1 && pl->split == 1 && cn.nq <= 6)
             take = cn.nq > 2 && elems >= (uint64_t(1) << 26);
         else if (bf16) take = pl->vec >= 2 || elems <= (uint64_t(1) << 24);
         else if (pl->rows_m == 1) take = elems >= (uint64_t(1) << 26) && cn.P >= 16;
@@ -462,6 +480,9 @@ void route_general(const Canon& cn, const void* a, const void* b, int sms, Plan*
     g.k.waq = cn.nq > 1 ? cn.P : 0;
     g.k.wb = 1;
     gs_plan(sms, &g);
+    // sums that the thin kernel spread over a slab's lanes, a row or two each: by exact steps
+    const uint64_t ways = (uint64_t)g.k.nseg << (g.k.wi_log2 + g.k.cluster_log2), rows = (BLOCK / 32) * (32 / std::max<uint64_t>(1, cn.P / pl->vec));
+    g.exact = !f64 && (pl->kind == KIND_COL_THIN || pl->small_slabs) && cn.nq <= 64 * ways && cn.nq <= (bf16 ? rows : 2 * rows);
     if (pl->kind == KIND_ROW && !f64 && !bf16 && pl->split == 1) {
         const uint64_t loads = cn.nq / g.V;   // whole blocks of four for every lane
         if (loads % (uint64_t(4) << g.k.group_log2) != 0) return;
@@ -895,11 +916,20 @@ int make_plan_inner(int dtype, const Canon& cn, const void* a, const void* b, co
             const uint64_t TO1 = (uint64_t)(BLOCK / 32) * 32 * V;
             Plan probe = pl;
             probe.group = 1;
-            thin = cdiv(outputs, TO1) < (uint64_t)sms * std::max(1, plan_ctas_per_sm(probe));
+            const bool few = cdiv(outputs, TO1) < (uint64_t)sms * std::max(1, plan_ctas_per_sm(probe));
+            thin = few;
             // a slab of less than one step of the CTA's warps leaves most of them idle; a CTA
             // per slab is still the shortest launch while each SM gets one at most (fp64 832
             // slabs of 4 x 4: 8.7 -> 3.4 us; 24 of 20 x 16 fp32 2.3, without it 2.7)
-            thin = thin && (cn.S <= (uint64_t)sms || cn.nq >= (BLOCK / 32) * (32 / PV));
+            // In fp32 and bf16 they then run on the general-stride kernels, which at up to four
+            // slabs per SM win where a few rows or many slabs leave the thin kernel's CTAs little
+            // (fp32 153 slabs of 64 x 5: 2.6 us, there 2.95; 2 x 64: 2.7, 3.1; 320 of 16 x 9 3.3,
+            // 2.9; bf16 256 of 2 x 32 2.8, 6.7, 1500 6.4, 10.6, 8000 21, 10.6).
+            const bool wave = cn.S <= 4 * (uint64_t)sms, wide = cn.P >= 8 || cn.P * cn.S >= (cn.nq > 128 ? 64 : 16) * (uint64_t)sms;
+            const bool gs_slabs = dtype == F64 ? true
+                                  : dtype == F32 ? !wave || cn.nq <= 4 || (cn.S >= 2 * (uint64_t)sms && cn.nq <= 64 && cn.nq * cn.P <= (uint64_t(1) << 11))
+                                                 : (wide || cn.nq <= 9) && (!wave || cn.nq < 100);
+            thin = thin && (cn.S <= (uint64_t)sms || cn.nq >= (BLOCK / 32) * (32 / PV) || !gs_slabs);
             // Many slabs: a CTA reduces through shared memory once per slab, which small slabs
             // do not pay for.  Column kernel from 4 slabs per SM on (fp64: also from one, where
             // a slab is long enough for its split): fp64 1000 slabs of 4 x 512 13.6 -> 8.7 us,
@@ -909,7 +939,8 @@ int make_plan_inner(int dtype, const Canon& cn, const void* a, const void* b, co
             if (dtype == F64)
                 thin = thin && !(cn.S > (uint64_t)sms && slab <= (1u << 15) && (cn.S >= 4 * (uint64_t)sms || slab >= (1u << 13)));
             else if (dtype == BF16A)
-                thin = thin && !(cn.S >= 4 * (uint64_t)sms && slab <= (1u << 12));
+                thin = thin && !(cn.S >= 4 * (uint64_t)sms && slab <= (1u << 12) && gs_slabs);
+            pl.small_slabs = few && !thin;
         }
         if (thin) {
             pl.kind = KIND_COL_THIN;

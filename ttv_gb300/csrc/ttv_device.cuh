@@ -154,6 +154,42 @@ __device__ __forceinline__ void kahan_pair(Acc<float, true>& p, Acc<float, true>
         : "f"(a0), "f"(a1), "f"(-b0), "f"(-b1));
 }
 
+// One exact step of a fp32 sum: the product's rounding error and that of the addition
+// (two-sum: the new term may be the larger one, which Kahan's step takes to be the
+// smaller) both go into c.  For the steps that start a sum, see GsSum::add; packed
+// for two sums as above, ten instructions for two elements.
+__device__ __forceinline__ void exact_step(Acc<float, true>& p, float a, float b)
+{
+    const float m = a * b, e = fmaf(-a, b, m);
+    p.merge(m, e);
+}
+__device__ __forceinline__ void exact_pair(Acc<float, true>& p, Acc<float, true>& q, float a0, float a1, float b0, float b1)
+{
+    // m = -(a b) rounded, f = a b + m its error; t = s - m, x the error of that sum
+    asm("{\n\t"
+        ".reg .b64 a, b, nb, s, c, m, f, t, d, x;\n\t"
+        "mov.b64 a, {%4, %5};\n\t"
+        "mov.b64 b, {%6, %7};\n\t"
+        "mov.b64 nb, {%8, %9};\n\t"
+        "mov.b64 s, {%0, %2};\n\t"
+        "mov.b64 c, {%1, %3};\n\t"
+        "mul.rn.f32x2 m, a, nb;\n\t"
+        "fma.rn.f32x2 f, a, b, m;\n\t"
+        "sub.rn.f32x2 t, s, m;\n\t"
+        "sub.rn.f32x2 d, t, s;\n\t"
+        "sub.rn.f32x2 x, t, d;\n\t"
+        "sub.rn.f32x2 x, s, x;\n\t"
+        "add.rn.f32x2 d, d, m;\n\t"
+        "sub.rn.f32x2 x, x, d;\n\t"
+        "sub.rn.f32x2 c, c, f;\n\t"
+        "sub.rn.f32x2 c, c, x;\n\t"
+        "mov.b64 {%0, %2}, t;\n\t"
+        "mov.b64 {%1, %3}, c;\n\t"
+        "}"
+        : "+f"(p.s), "+f"(p.c), "+f"(q.s), "+f"(q.c)
+        : "f"(a0), "f"(a1), "f"(b0), "f"(b1), "f"(-b0), "f"(-b1));
+}
+
 // acc[n] += x[n] y[n].  PAIR off: where a sum starts in straight-line code, whose first
 // product the compiler fuses into the second step's addition (a rounding less, which
 // sums of a few terms show: 4 rows 2.9e-8, in packed steps 3.6e-8).
@@ -167,6 +203,14 @@ __device__ __forceinline__ void fma_add_all(AccT (&acc)[N], const T (&x)[N], con
 #pragma unroll
         for (int n = 0; n < N; ++n) acc[n].fma_add(x[n], y[n]);
     }
+}
+
+// The same in exact steps.
+template <int N> __device__ __forceinline__ void exact_add_all(Acc<float, true> (&acc)[N], const float (&x)[N], const float (&y)[N])
+{
+#pragma unroll
+    for (int n = 0; n + 1 < N; n += 2) exact_pair(acc[n], acc[n + 1], x[n], x[n + 1], y[n], y[n + 1]);
+    if constexpr (N % 2) exact_step(acc[N - 1], x[N - 1], y[N - 1]);
 }
 
 // --------------------------------------------------------------------------

@@ -191,28 +191,41 @@ __device__ __noinline__ double2 fx_fold(uint4 w, int base, double s, double c)
 // the dense kernels' mix of native and double-float products.
 template <typename T, int N, int SUM> struct GsSum {
     Acc<T, true> acc[N];
-    bool fresh;
-    __device__ __forceinline__ void init()
+    uint32_t lead;   // blocks that start the sum
+    __device__ __forceinline__ void init(uint32_t blocks)
     {
 #pragma unroll
         for (int n = 0; n < N; ++n) acc[n].init();
-        fresh = true;
+        lead = SUM == GS_EXACT ? blocks : 1u;
     }
-    // x[u][n] y[u][n] into output n; PART: only those with u < count.  GS_FIRST: the
-    // first product goes in exactly (rounded value and its error), which a sum of
-    // few terms shows (4 rows: rms error 3.6e-8 -> 2.9e-8), and the kernels got faster
-    // for it (512^3 bf16 50.3 -> 44.3 us, 256^3 fp32 13.2 -> 12.2, 64 x 64 x 4096
-    // 14.4 -> 12.8); bf16 rows in 16-byte loads would spill (26.7 -> 43.5 us).
+    // x[u][n] y[u][n] into output n; PART: only those with u < count.  A sum's first
+    // terms are where Kahan's steps lose, as the next term is often larger than the sum
+    // so far.  GS_FIRST: the first product goes in exactly (its rounded value and its
+    // error), and the kernels got faster for it (512^3 bf16 50.3 -> 44.3 us, 256^3 fp32
+    // 13.2 -> 12.2, 64 x 64 x 4096 14.4 -> 12.8; bf16 rows in 16-byte loads would spill:
+    // 26.7 -> 43.5 us).  GS_EXACT: the first block, of short sums the first two, by
+    // exact steps (one such block cost the long sums of bf16 columns 7 %).
     template <bool PART, int UB>
     __device__ __forceinline__ void add(const T (&x)[UB][N], const T (&y)[UB][N], int count)
     {
-        if (SUM == GS_FIRST && fresh) {
+        if constexpr (SUM == GS_EXACT) {
+            if (lead > 0) {
+                --lead;
+#pragma unroll
+                for (int u = 0; u < UB; ++u) {
+                    if (PART && u > 0 && u >= count) break;
+                    exact_add_all<N>(acc, x[u], y[u]);
+                }
+                return;
+            }
+        }
+        if (SUM == GS_FIRST && lead) {
 #pragma unroll
             for (int n = 0; n < N; ++n) {
                 acc[n].s = x[0][n] * y[0][n];
                 acc[n].c = fma(-x[0][n], y[0][n], acc[n].s);
             }
-            fresh = false;
+            lead = 0;
         } else {
             fma_add_all<N>(acc, x[0], y[0]);
         }
@@ -228,7 +241,7 @@ template <typename T, int N, int SUM> struct GsSum {
 template <int N> struct GsSum<double, N, GS_FX> {
     FxAcc acc[N];
     int base, budget;
-    __device__ __forceinline__ void init()
+    __device__ __forceinline__ void init(uint32_t)
     {
 #pragma unroll
         for (int n = 0; n < N; ++n) fx_init(acc[n]);
@@ -320,7 +333,7 @@ template <int N> struct GsSum<double, N, GS_FX> {
 };
 template <int N> struct GsSum<double, N, GS_MIX> {
     AccDF acc[N];
-    __device__ __forceinline__ void init()
+    __device__ __forceinline__ void init(uint32_t)
     {
 #pragma unroll
         for (int n = 0; n < N; ++n) acc[n].init();
@@ -529,7 +542,7 @@ __global__ void __launch_bounds__(256, gs_col_ctas<T, V * MO, SHARE>()) gs_col_k
             rows = i < i1 ? ((i1 - i - 1) >> wl) + 1 : 0;
         }
         GsSum<T, N, SUM> sum;
-        sum.init();
+        sum.init(k.lead);
         uint64_t co[MO];
         const TA* rp[MO];
 #pragma unroll
@@ -628,7 +641,7 @@ __global__ void __launch_bounds__(256, gs_row_ctas<T>()) gs_row_kernel(GSArgs k)
         const uint64_t nv = (i1 - i0) / V;   // V divides every range
         const uint64_t first = ((uint64_t)wi << k.group_log2) + gl;   // the lane's first vector of the range
         GsSum<T, N, SUM> sum;
-        sum.init();
+        sum.init(k.lead);
         uint64_t co[R];
         const TA* rp[R];
 #pragma unroll
@@ -741,20 +754,20 @@ void gs_modes(std::vector<std::tuple<size_t, size_t, size_t>> modes, GSArgs* k)
 // The plan's kernel, and the loads each of its lanes keeps in flight per row or
 // vector of outputs (U).
 typedef void (*GsFn)(GSArgs);
-template <bool SHARE> static GsFn gs_kernel_of(const GSPlan& p, int& U)
+template <bool SHARE, int SUM> static GsFn gs_kernel_of(const GSPlan& p, int& U)
 {
     const int M = p.M;
     if (p.dtype == BF16A) {
         if (p.row) {
             U = p.V > 1 ? 4 : 8 / M;
             if (p.V > 1) return gs_row_kernel<uint16_t, float, 8, 1, 4, GS_KAHAN, SHARE>;
-            return M == 4 ? gs_row_kernel<uint16_t, float, 1, 4, 2, GS_FIRST, SHARE>
-                          : (M == 2 ? gs_row_kernel<uint16_t, float, 1, 2, 4, GS_FIRST, SHARE> : gs_row_kernel<uint16_t, float, 1, 1, 8, GS_FIRST, SHARE>);
+            return M == 4 ? gs_row_kernel<uint16_t, float, 1, 4, 2, SUM, SHARE>
+                          : (M == 2 ? gs_row_kernel<uint16_t, float, 1, 2, 4, SUM, SHARE> : gs_row_kernel<uint16_t, float, 1, 1, 8, SUM, SHARE>);
         }
         U = p.V == 8 ? 4 : 8;
-        if (p.V == 8) return gs_col_kernel<uint16_t, float, 8, 1, 4, GS_FIRST, SHARE>;
-        if (p.V == 2) return gs_col_kernel<uint16_t, float, 2, 2, 8, GS_FIRST, SHARE>;
-        return M == 2 ? gs_col_kernel<uint16_t, float, 1, 2, 8, GS_FIRST, SHARE> : gs_col_kernel<uint16_t, float, 1, 1, 8, GS_FIRST, SHARE>;
+        if (p.V == 8) return gs_col_kernel<uint16_t, float, 8, 1, 4, SUM, SHARE>;
+        if (p.V == 2) return gs_col_kernel<uint16_t, float, 2, 2, 8, SUM, SHARE>;
+        return M == 2 ? gs_col_kernel<uint16_t, float, 1, 2, 8, SUM, SHARE> : gs_col_kernel<uint16_t, float, 1, 1, 8, SUM, SHARE>;
     }
     if (p.dtype == F64 && p.mix) {
         U = p.V > 1 ? 4 : 8;
@@ -780,19 +793,20 @@ template <bool SHARE> static GsFn gs_kernel_of(const GSPlan& p, int& U)
     }
     if (p.row) {
         U = p.V > 1 ? 4 / M : 8 / M;
-        if (p.V > 1) return M == 2 ? gs_row_kernel<float, float, 4, 2, 2, GS_FIRST, SHARE> : gs_row_kernel<float, float, 4, 1, 4, GS_FIRST, SHARE>;
-        return M == 4 ? gs_row_kernel<float, float, 1, 4, 2, GS_FIRST, SHARE>
-                      : (M == 2 ? gs_row_kernel<float, float, 1, 2, 4, GS_FIRST, SHARE> : gs_row_kernel<float, float, 1, 1, 8, GS_FIRST, SHARE>);
+        if (p.V > 1) return M == 2 ? gs_row_kernel<float, float, 4, 2, 2, SUM, SHARE> : gs_row_kernel<float, float, 4, 1, 4, SUM, SHARE>;
+        return M == 4 ? gs_row_kernel<float, float, 1, 4, 2, SUM, SHARE>
+                      : (M == 2 ? gs_row_kernel<float, float, 1, 2, 4, SUM, SHARE> : gs_row_kernel<float, float, 1, 1, 8, SUM, SHARE>);
     }
     U = p.V > 1 ? 4 / M : (M == 4 ? 4 : 8);
-    if (p.V > 1) return M == 2 ? gs_col_kernel<float, float, 4, 2, 2, GS_FIRST, SHARE> : gs_col_kernel<float, float, 4, 1, 4, GS_FIRST, SHARE>;
-    return M == 4 ? gs_col_kernel<float, float, 1, 4, 4, GS_FIRST, SHARE>
-                  : (M == 2 ? gs_col_kernel<float, float, 1, 2, 8, GS_FIRST, SHARE> : gs_col_kernel<float, float, 1, 1, 8, GS_FIRST, SHARE>);
+    if (p.V > 1) return M == 2 ? gs_col_kernel<float, float, 4, 2, 2, SUM, SHARE> : gs_col_kernel<float, float, 4, 1, 4, SUM, SHARE>;
+    return M == 4 ? gs_col_kernel<float, float, 1, 4, 4, SUM, SHARE>
+                  : (M == 2 ? gs_col_kernel<float, float, 1, 2, 8, SUM, SHARE> : gs_col_kernel<float, float, 1, 1, 8, SUM, SHARE>);
 }
 static GsFn gs_kernel(const GSPlan& p, bool share, int* u = nullptr)
 {
     int U = 1;
-    const GsFn fn = share ? gs_kernel_of<true>(p, U) : gs_kernel_of<false>(p, U);
+    const GsFn fn = p.exact ? (share ? gs_kernel_of<true, GS_EXACT>(p, U) : gs_kernel_of<false, GS_EXACT>(p, U))
+                            : (share ? gs_kernel_of<true, GS_FIRST>(p, U) : gs_kernel_of<false, GS_FIRST>(p, U));
     if (u) *u = U;
     return fn;
 }
@@ -870,6 +884,7 @@ static void gs_split(GSPlan* p, uint64_t rows, bool may_split, bool segments, ui
     k.tiles = tiles(k.wi_log2);
     k.items = k.tiles * k.nseg;
     k.tdiv = make_idx_div(k.tiles, k.items);
+    k.lead = rows <= 64 * ((uint64_t)k.nseg << (k.wi_log2 + k.cluster_log2)) ? 2 : 1;
     // a CTA (cluster) per item, which the hardware levels; beyond 32 per SM round robin
     p->grid = (int)(std::min<uint64_t>(k.items, ((uint64_t)sms * 32) >> k.cluster_log2) << k.cluster_log2);
 }

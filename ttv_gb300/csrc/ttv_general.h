@@ -32,11 +32,12 @@ struct GSArgs {
     uint32_t cluster_log2;        // CTAs of a cluster, all along q
     uint32_t wi_log2;             // warps along q
     uint32_t group_log2;          // row form: lanes per output
+    uint32_t lead;                // fp32 sums: blocks added by exact steps (GS_EXACT)
 };
 
 // How a thread sums: Kahan, fp64 products in fixed point, fp64 native and double-float products,
-// fp32 Kahan whose first product is exact.
-enum GsMode { GS_KAHAN = 0, GS_FX = 1, GS_MIX = 2, GS_FIRST = 3 };
+// fp32 Kahan whose first product is exact, fp32 Kahan whose first block of products is.
+enum GsMode { GS_KAHAN = 0, GS_FX = 1, GS_MIX = 2, GS_FIRST = 3, GS_EXACT = 4 };
 
 struct GSPlan {
     GSArgs k{};
@@ -44,6 +45,7 @@ struct GSPlan {
     bool row = false;
     bool fx = false;        // fp64: fixed-point sums (else Kahan)
     bool mix = false;       // fp64, set by the caller: the dense kernels' mixed products instead
+    bool exact = true;      // fp32, bf16: first block of a sum exact (else its first product)
     int V = 1, M = 1;       // vector width; vectors per thread (column) or rows per group (row)
     int grid = 1;
 };

@@ -82,6 +82,7 @@ struct Plan {
     int stream_col = 0;          // 0: row form (P == 1), 1: column form
     uint64_t L = 0, R = 0, units = 0, units_per_cta = 0;
     int RG = 1, J = 1;
+    bool small_slabs = false;    // COL: few outputs, but slabs too short or too many for the thin kernel
     // ROW / COL: runs on the general-stride kernels (ttv_general.cu), `gs` its plan
     bool general = false;
     GSPlan gs;
