@@ -945,6 +945,7 @@ int make_plan_inner(int dtype, const Canon& cn, const void* a, const void* b, co
         if (thin) {
             pl.kind = KIND_COL_THIN;
             pl.group = 1;
+            pl.rows_m = thin_ragged ? 1 : 0;
             const int cps = std::max(1, plan_ctas_per_sm(pl));
             const uint64_t grid_full = (uint64_t)sms * cps;
             const uint64_t RG = 32 / PV;
@@ -955,8 +956,13 @@ int make_plan_inner(int dtype, const Canon& cn, const void* a, const void* b, co
                     return fail(TLIBG_ERR_ARGUMENT, "tlibg: forced split leaves a segment longer than the staged b buffer");
                 nseg = (uint64_t)force_split;
             } else if (cn.S * nseg < 2 * grid_full) {
+                const uint64_t least = nseg;
                 nseg = std::max<uint64_t>(nseg, std::min<uint64_t>(cdiv(2 * grid_full, cn.S),
                                                                    std::max<uint64_t>(1, cn.nq / min_len)));
+                // bf16, items a little over one wave: one wave of longer ones (16-byte loads with packed
+                // steps hold four CTAs per SM, without them five: 40 slabs of 8 x 20000 11.0 -> 12.0 us)
+                if (dtype == BF16A && cn.S * nseg > grid_full && 2 * cn.S * nseg < 3 * grid_full && cn.S <= grid_full)
+                    nseg = std::max<uint64_t>(least, grid_full / cn.S);
             }
             nseg = std::max<uint64_t>(1, std::min<uint64_t>(nseg, cn.nq));
             const uint64_t seg_len = cdiv(cn.nq, nseg);

@@ -182,9 +182,10 @@ template <int V, typename AccT> __device__ __forceinline__ void renorm_all(AccT 
 // mix when V == 1).
 // rp points at the thread's vector in row i and moves on by `step` elements
 // (WI rows) per row: one pointer add per load.
-template <int UB, int V, bool PRE = false, typename TA, typename T, typename AccT>
+// START: by exact steps while `lead` (the sum's first block).
+template <int UB, int V, bool PRE = false, bool START = false, typename TA, typename T, typename AccT>
 __device__ __forceinline__ void col_rows(AccT (&acc)[V], const TA*& rp, uint64_t step, const T* bs, uint64_t i,
-                                         uint32_t WI, const float2* bsp = nullptr)
+                                         uint32_t WI, const float2* bsp, bool& lead)
 {
     T av[UB][V];
 #pragma unroll
@@ -192,34 +193,49 @@ __device__ __forceinline__ void col_rows(AccT (&acc)[V], const TA*& rp, uint64_t
         load_a<TA, T, V>(rp, av[u]);
         rp += step;
     }
+    if constexpr (START) {
+        if (lead) {
 #pragma unroll
-    for (int u = 0; u < UB; ++u) row_fma<V, PRE>(acc, av[u], bs[i + u * WI], u, PRE ? bsp + i + u * WI : nullptr);
+            for (int u = 0; u < UB; ++u) {
+                T bv[V];
+#pragma unroll
+                for (int v = 0; v < V; ++v) bv[v] = bs[i + u * WI];
+                exact_add_all<V>(acc, av[u], bv);
+            }
+            lead = false;
+            return;
+        }
+    }
+#pragma unroll
+    for (int u = 0; u < UB; ++u)
+        row_fma<V, PRE>(acc, av[u], bs[i + u * WI], u, PRE ? bsp + i + u * WI : nullptr);
     renorm_all<V>(acc);
 }
 
 // Rows [i0, ie) step WI of one thread: blocks of U rows, then one of U/2 and
 // one of U/4 at most, then single rows, so short contractions still get
 // their loads in flight together.
-template <int U, int V, bool PRE, typename TA, typename T, typename AccT>
+template <int U, int V, bool PRE, bool START = false, typename TA, typename T, typename AccT>
 __device__ __forceinline__ void col_loop(AccT (&acc)[V], const TA* ap, uint64_t P, const T* bs, const float2* bsp,
                                          uint64_t i, uint64_t ie, uint32_t WI)
 {
     const TA* rp = ap + i * P;
     const uint64_t step = uint64_t(WI) * P;
-    for (; i + (U - 1) * WI < ie; i += U * WI) col_rows<U, V, PRE>(acc, rp, step, bs, i, WI, bsp);
+    bool lead = START;
+    for (; i + (U - 1) * WI < ie; i += U * WI) col_rows<U, V, PRE, START>(acc, rp, step, bs, i, WI, bsp, lead);
     if constexpr (U >= 4) {
         if (i + (U / 2 - 1) * WI < ie) {
-            col_rows<U / 2, V, PRE>(acc, rp, step, bs, i, WI, bsp);
+            col_rows<U / 2, V, PRE, START>(acc, rp, step, bs, i, WI, bsp, lead);
             i += (U / 2) * WI;
         }
     }
     if constexpr (U >= 8) {
         if (i + (U / 4 - 1) * WI < ie) {
-            col_rows<U / 4, V, PRE>(acc, rp, step, bs, i, WI, bsp);
+            col_rows<U / 4, V, PRE, START>(acc, rp, step, bs, i, WI, bsp, lead);
             i += (U / 4) * WI;
         }
     }
-    for (; i < ie; i += WI) col_rows<1, V, PRE>(acc, rp, step, bs, i, WI, bsp);
+    for (; i < ie; i += WI) col_rows<1, V, PRE, START>(acc, rp, step, bs, i, WI, bsp, lead);
 }
 
 // fp64 with the double-float mix: b's split is computed once per staged
@@ -260,7 +276,8 @@ __device__ __forceinline__ void row_vecs(AccT (&acc)[V], const TA* ap, const T* 
         load_b<T, V>(bp + (kv + u * G) * V, bv[u]);
     }
 #pragma unroll
-    for (int u = 0; u < UB; ++u) vec_fma<V, PRE>(acc, av[u], bv[u], u, PRE ? bsp + (kv + u * G) * V : nullptr);
+    for (int u = 0; u < UB; ++u)
+        vec_fma<V, PRE>(acc, av[u], bv[u], u, PRE ? bsp + (kv + u * G) * V : nullptr);
     renorm_all<V>(acc);
 }
 
@@ -830,10 +847,10 @@ static KernelFn pick_main(int kind, int vec, int rows_m, int mo)
     }
     if (kind == KIND_COL_THIN) {
         switch (vec) {
-        case 1: return col_thin_kernel<TA, T, 1, KAHAN>;
-        case 2: return col_thin_kernel<TA, T, 2, KAHAN>;
-        case 4: if constexpr (VMAX >= 4) return col_thin_kernel<TA, T, 4, KAHAN>; else return nullptr;
-        case 8: if constexpr (VMAX >= 8) return col_thin_kernel<TA, T, 8, KAHAN>; else return nullptr;
+        case 1: return rows_m ? col_thin_kernel<TA, T, 1, KAHAN, true> : col_thin_kernel<TA, T, 1, KAHAN, false>;
+        case 2: return rows_m ? col_thin_kernel<TA, T, 2, KAHAN, true> : col_thin_kernel<TA, T, 2, KAHAN, false>;
+        case 4: if constexpr (VMAX >= 4) return rows_m ? col_thin_kernel<TA, T, 4, KAHAN, true> : col_thin_kernel<TA, T, 4, KAHAN, false>; else return nullptr;
+        case 8: if constexpr (VMAX >= 8) return rows_m ? col_thin_kernel<TA, T, 8, KAHAN, true> : col_thin_kernel<TA, T, 8, KAHAN, false>; else return nullptr;
         }
         return nullptr;
     }

@@ -11,13 +11,23 @@
 // The 8 warps of a CTA interleave along the contracted mode; a work item is
 // one (segment of q, slab s).  Lanes of the same outputs are reduced by
 // shuffles, the warps through shared memory in fixed order, segments by the
-// deterministic combine kernel.  Every lane is busy whatever P and S are.
+// deterministic combine kernel.
 #pragma once
 
 namespace tlibg {
 
-template <typename TA, typename T, int V, bool KAHAN>
-__global__ void __launch_bounds__(BLOCK, (min_ctas<TA, V>())) col_thin_kernel(KArgs k)
+// Resident CTAs per SM: as the other register kernels for 16-byte loads, three for narrower
+// ones (bf16 in 8-byte loads needs 84 registers else, two CTAs: 400 slabs of 4 x 100 3.9 -> 4.6 us).
+template <typename TA, int V> __host__ __device__ constexpr int thin_ctas()
+{
+    return (int)sizeof(TA) * V >= 16 ? min_ctas<TA, V>() : 3;
+}
+
+// RAGGED: P / V does not divide 32.  A kernel of its own: the reduction over idle lanes and the
+// exact start in one kernel with the whole warps' cost those 3 to 20 % (1900 x 32 fp32
+// 4.35 -> 5.3 us, 16384 slabs of 4 x 512 65.6 -> 70.9).
+template <typename TA, typename T, int V, bool KAHAN, bool RAGGED>
+__global__ void __launch_bounds__(BLOCK, (thin_ctas<TA, V>())) col_thin_kernel(KArgs k)
 {
     pdl_prologue();
     constexpr int NW = BLOCK / 32;
@@ -38,7 +48,6 @@ __global__ void __launch_bounds__(BLOCK, (min_ctas<TA, V>())) col_thin_kernel(KA
     const uint32_t PV = (uint32_t)(P / V);   // lanes per row
     const uint32_t RG = 32u / PV;            // rows per warp step
     const uint32_t g = lane / PV;            // row group; RG: an idle lane
-    const bool whole = PV * RG == 32u;       // every lane works
     const uint64_t j0 = (uint64_t)(lane % PV) * V;
     const uint32_t step = NW * RG;           // rows between a lane's consecutive loads
     const TA* __restrict__ A = static_cast<const TA*>(k.a);
@@ -76,19 +85,21 @@ __global__ void __launch_bounds__(BLOCK, (min_ctas<TA, V>())) col_thin_kernel(KA
 #pragma unroll
         for (int v = 0; v < V; ++v) acc[v].init();
         const TA* ap = A + s * k.nq * P + j0;
-        const uint64_t i0 = g < RG ? ib + warp * RG + g : ie;
+        const uint64_t i0 = !RAGGED || g < RG ? ib + warp * RG + g : ie;
         if constexpr (PRES) {
             if (b_split_ok)
                 col_loop<U, V, true>(acc, ap, P, bs, bsp, i0, ie, step);
             else
                 col_loop<U, V, false>(acc, ap, P, bs, bsp, i0, ie, step);
         } else {
-            col_loop<U, V, false>(acc, ap, P, bs, bsp, i0, ie, step);
+            // ragged: in place of a column-kernel split of fewer, longer sums, whose error
+            // these keep by an exact start (3 x 394 x 39 bf16: 2.54e-9, else 2.60e-9 rms)
+            col_loop<U, V, false, RAGGED && KAHAN>(acc, ap, P, bs, bsp, i0, ie, step);
         }
 #pragma unroll
         for (int v = 0; v < V; ++v) acc[v].fold();
         // lanes of the same outputs (row groups g) in the warp, then the warps
-        if (whole) {
+        if constexpr (!RAGGED) {
             for (uint32_t o = PV; o < 32u; o <<= 1) {
 #pragma unroll
                 for (int v = 0; v < V; ++v) {
