@@ -1081,7 +1081,8 @@ def test_error_of_short_sums(engine, cuda, P, nq, S, dtype):
     assert err <= 1.03 ** 2 * bar, (err / bar) ** 0.5
 
 
-@pytest.mark.parametrize("P,nq,S,dtype", [(3, 394, 39, "bf16"), (12, 194, 2, "bf16"), (24, 394, 6, "bf16"), (40, 100, 3, "bf16"),
+@pytest.mark.parametrize("P,nq,S,dtype", [(1, 257, 20000, "f32"), (1, 501, 20000, "f32"), (1, 721, 20000, "f32"), (1, 257, 20000, "bf16"),
+                                          (3, 394, 39, "bf16"), (12, 194, 2, "bf16"), (24, 394, 6, "bf16"), (40, 100, 3, "bf16"),
                                           (3, 5000, 4, "f32"), (24, 900, 2, "f32")])
 def test_error_of_rows_and_ragged_prefixes(engine, cuda, P, nq, S, dtype):
     """Row-shift rows and thin prefixes with idle lanes, many short sums per output: rms within
