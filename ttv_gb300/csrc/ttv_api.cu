@@ -769,16 +769,18 @@ int make_plan_inner(int dtype, const Canon& cn, const void* a, const void* b, co
     //     too where the row kernel would split them (over 64 long: 128 x 30000: 15.6 -> 9.1 us,
     //     512 x 1000: 6.4 -> 4.3, 1024 x 100000: 147 -> 134, 100 x 8: 4.8 -> 3.3; level
     //     where it would not); rows off it that would leave a second round of lane groups under
-    //     half full also stay with the unsplit row kernel (645 x 26011: 29.5, here 31.7);
+    //     half full also stay with the unsplit row kernel (645 x 26011: 29.5, here 31.7), and a
+    //     second round under a tenth full with its split too (1001 x 20000: 39.6, here 45.3);
     //   bf16: as fp32, rows of odd length and of 4-byte alignment from 256 elements
     //     (255 x 263172: 99 -> 37 us, 274 x 200000: 42 -> 30; 102 x 600000: 43.8 -> 47),
     //     up to 1024 (the eight copies of b take 32 bytes per element).
     Plan shift;
     bool shift_last = false;
+    uint64_t shift_groups = 0;
     if (shift_ok && (rows_aligned ? dtype == F64 && pl.kahan && cn.nq > 64 : cn.nq >= 64) && no_split && !(opt && (opt->kind >= 0 || opt->vec > 0)) &&
         make_row_shift_plan(pl, cn, opt, sms, &shift) == TLIBG_OK) {
         const uint64_t ctas = (uint64_t)sms * std::max(1, plan_ctas_per_sm(shift));
-        const uint64_t groups = ctas * (BLOCK / shift.group);
+        const uint64_t groups = shift_groups = ctas * (BLOCK / shift.group);
         bool take;
         if (opt && opt->group > 0) take = !rows_aligned && dtype != BF16A && cn.S >= 4 * groups;
         else if (dtype == F64) take = cn.nq <= 512 || cn.S >= (rows_aligned ? 512 : 256);
@@ -874,7 +876,7 @@ int make_plan_inner(int dtype, const Canon& cn, const void* a, const void* b, co
                     nseg = ns;
         }
         nseg = std::max<uint64_t>(1, std::min<uint64_t>(nseg, cn.nq));
-        if (shift_last && nseg > 1) {
+        if (shift_last && nseg > 1 && !(cn.S > shift_groups && 10 * cn.S < 11 * shift_groups && !rows_aligned)) {
             *out = shift;
             return TLIBG_OK;
         }
