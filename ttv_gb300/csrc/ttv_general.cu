@@ -861,7 +861,8 @@ static void gs_split(GSPlan* p, uint64_t rows, bool may_split, bool segments, ui
             if (segments && wl == 3 && cl == 3 && ctas < cap) ns = std::max<uint64_t>(1, std::min<uint64_t>(cap / ctas, rows / (64 * 16)));
             const uint64_t ways = (uint64_t)(1u << (wl + cl)) * ns;
             if (ways > 1 && (!may_split || rows < 2 * ways)) continue;
-            const double fixed = 1500 + (wl ? (p->mix ? 3000 : 5000) : 0) + (cl ? (p->mix ? 5000 : 6000) : 0) + (ns > 1 ? 6000 : 0);
+            // (launches of at most a CTA per SM pay half for sharing over warps)
+            const double fixed = 1500 + (wl ? (p->mix ? 3000 : tiles(wl) <= (uint64_t)sms && p->dtype != F64 ? 2500 : 5000) : 0) + (cl ? (p->mix ? 5000 : 6000) : 0) + (ns > 1 ? 6000 : 0);
             const double n = (double)up(ctas * ns, (uint64_t)sms), r = (double)up(rows, ways);
             const double chain = std::ceil(n / cps) * (std::ceil(r / U) * 1400 + fixed);
             // fp64 fixed point: turning a sum into a pair, and FP64 instructions per merge
@@ -931,8 +932,10 @@ void gs_plan(int sms, GSPlan* p, bool segments)
         auto columns = [&](uint64_t v) { return k.wa[0] == 1 && k.ext[0].d % v == 0 && k.waq % v == 0 && on_grid(v); };
         p->V = !plain && columns(V) ? (int)V : 1;
         // 16-byte vectors only while they leave a warp on every scheduler: the
-        // contracted mode is shared 64 ways at most before the grid is split
-        if (p->V > 1 && k.outputs / V * std::min<uint64_t>(64, std::max<uint64_t>(1, k.nq / 8)) < lanes / 2) p->V = 1;
+        // contracted mode is shared 64 ways at most before the grid is split, and not
+        // at all below 64 rows, whose chains end before sharing them pays (a view of
+        // 100 x 30 x 1000 4.3 -> 5.9 us in vectors)
+        if (p->V > 1 && k.outputs / V * (k.nq < 64 ? 1 : std::min<uint64_t>(64, k.nq / 8)) < lanes / 2) p->V = 1;
         if (bf16 && p->V == 1 && columns(2)) {
             p->V = p->M = 2;   // 4-byte loads, two vectors per thread
         } else if (p->V > 1) {
