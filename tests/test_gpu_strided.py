@@ -353,3 +353,94 @@ def test_captured_scratch_outlives_its_growth(engine, cuda):
     torch.cuda.synchronize()
     check()
     assert engine.device_error() == 0
+
+
+# (outputs, contraction): shared by warps and clusters, and a thread's own; more than 1500 products per SM,
+# from where fp64 views are summed in fixed point
+FX_SHAPES = [(401, 3000), (60003, 37)]
+
+
+def _fx_view(torch, a, cuda, form, wide):
+    """a's view with the contracted mode second: `row` as its fastest mode, `col` as its slower
+    one, on the 16-byte grid (`wide`) and off it."""
+    t = torch.from_numpy(np.ascontiguousarray(a if form == "row" else a.T)).to(cuda)
+    pad = 2 - t.shape[1] % 2 if wide else 1 + t.shape[1] % 2
+    t = torch.nn.functional.pad(t, (0, pad))[:, :t.shape[1]]
+    return t if form == "row" else t.T
+
+
+@pytest.mark.parametrize("wide", [True, False], ids=["vectors", "elements"])
+@pytest.mark.parametrize("form", ["row", "col"])
+@pytest.mark.parametrize("shape", FX_SHAPES, ids=["shared", "own"])
+@pytest.mark.parametrize("kind", ["growing", "falling", "zeros", "negative_zeros", "huge", "tiny", "mixed", "cancelling", "negative"])
+def test_fp64_fixed_point_sums(engine, cuda, kind, shape, form, wide):
+    """The fixed-point kernels themselves (enough products per SM): moving bases, products below the
+    window, zeros of both signs, the ends of the exponent range, cancellation, negative sums.  Bar: one
+    rounding per product and the result's, of sum |a b|, and of the smallest number per product."""
+    import fractions
+    import torch
+    m, n = shape
+    assert m * n > 1500 * torch.cuda.get_device_properties(0).multi_processor_count and n >= 4
+    rng = np.random.default_rng(12)
+    a = rng.uniform(-1, 1, (m, n))
+    if kind == "growing":
+        a *= np.exp2(np.linspace(-300, 300, n))
+    elif kind == "falling":
+        a *= np.exp2(np.linspace(300, -300, n))
+    elif kind in ("zeros", "negative_zeros"):
+        a[rng.uniform(size=a.shape) < 0.5] = 0.0 if kind == "zeros" else -0.0
+        a[5], a[m - 1] = 0.0, -0.0
+        a[7, :-1] = 0.0
+    elif kind == "huge":
+        a *= 2.0 ** 1009
+    elif kind == "tiny":
+        a *= 2.0 ** -1020
+    elif kind == "mixed":
+        a *= np.exp2(rng.uniform(-200, 200, a.shape))
+    elif kind == "cancelling":
+        a[:, 1:n // 2 * 2:2] = -a[:, 0:n // 2 * 2:2]
+    else:
+        a = -np.abs(a)
+    b = np.ones(n) if kind == "cancelling" else rng.uniform(0.25, 1, n) if kind == "negative" else rng.uniform(-1, 1, n)
+    c = engine.ttv_view(2, _fx_view(torch, a, cuda, form, wide), torch.from_numpy(b).to(cuda)).cpu().numpy()
+    bs = [fractions.Fraction(y) for y in b]
+    for i in sorted({0, 5, 7, m - 1, *range(1, m, 40 if n > 1000 else 600)}):
+        terms = [fractions.Fraction(x) * y for x, y in zip(a[i], bs)]
+        exact, absn = sum(terms), sum(abs(t) for t in terms)
+        bar = absn * fractions.Fraction(4, 2 ** 53) + n * fractions.Fraction(1, 2 ** 1074)
+        assert abs(fractions.Fraction(float(c[i])) - exact) <= bar, (kind, i)
+
+
+@pytest.mark.parametrize("wide", [True, False], ids=["vectors", "elements"])
+@pytest.mark.parametrize("form", ["row", "col"])
+@pytest.mark.parametrize("shape", FX_SHAPES, ids=["shared", "own"])
+def test_fp64_fixed_point_nonfinite(engine, cuda, shape, form, wide):
+    """Infinities and NaNs among many products reach their output and no other."""
+    import torch
+    rng = np.random.default_rng(13)
+    m, n = shape
+    a, b = rng.uniform(-1, 1, shape), rng.uniform(0.5, 1, n)
+    bad = np.zeros(m, bool)
+    for i, v in ((3, np.inf), (8, np.nan), (20, -np.inf), (m - 1, np.inf), (m // 2, 1.7e308)):
+        a[i, (i * 5) % n] = v
+        bad[i] = True
+    a[m // 2, :3] = 1.7e308
+    c = engine.ttv_view(2, _fx_view(torch, a, cuda, form, wide), torch.from_numpy(b).to(cuda)).cpu().numpy()
+    assert (np.isfinite(c) == ~bad).all()
+    assert np.abs(c[~bad] - a[~bad] @ b).max() <= 1e-13 * n
+
+
+def test_fp64_fixed_point_folds_in_time(engine, cuda):
+    """A thread's sum of more products than the fixed-point accumulator holds between folds (2^18):
+    one row of A broadcast over enough outputs that no two threads share a sum."""
+    import fractions
+    import torch
+    rng = np.random.default_rng(14)
+    n, m = (1 << 18) + 1003, 2048 * torch.cuda.get_device_properties(0).multi_processor_count
+    a, b = rng.uniform(0.5, 1, n), rng.uniform(0.5, 1, n)
+    a[1::2] *= -0.25
+    c = engine.ttv_view(2, torch.from_numpy(a).to(cuda).expand(m, n), torch.from_numpy(b).to(cuda))
+    terms = [fractions.Fraction(x) * fractions.Fraction(y) for x, y in zip(a, b)]
+    exact, absn = sum(terms), sum(abs(t) for t in terms)
+    assert (c == c[0]).all()
+    assert abs(fractions.Fraction(float(c[0])) - exact) <= absn * fractions.Fraction(4, 2 ** 53)

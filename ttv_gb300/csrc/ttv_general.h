@@ -35,9 +35,9 @@ struct GSArgs {
     uint32_t lead;                // fp32 sums: blocks added by exact steps (GS_EXACT)
 };
 
-// How a thread sums: Kahan, fp64 products in fixed point, fp64 native and double-float products,
+// How a thread sums: Kahan, fp64 products in fixed point (columns, rows), fp64 native and double-float products,
 // fp32 Kahan whose first product is exact, fp32 Kahan whose first block of products is.
-enum GsMode { GS_KAHAN = 0, GS_FX = 1, GS_MIX = 2, GS_FIRST = 3, GS_EXACT = 4 };
+enum GsMode { GS_KAHAN = 0, GS_FX = 1, GS_MIX = 2, GS_FIRST = 3, GS_EXACT = 4, GS_FX_ROW = 5 };
 
 struct GSPlan {
     GSArgs k{};
