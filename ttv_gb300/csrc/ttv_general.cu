@@ -927,8 +927,10 @@ void gs_plan(int sms, GSPlan* p, bool segments)
     };
     const uint64_t V = 16 / ea;
     // fp64: Kahan sums (four FP64 instructions an element against one, but a tenth of
-    // the code) while all of them together are about a microsecond of the FP64 pipes
-    p->fx = f64 && !p->mix && k.outputs * k.nq > (uint64_t)sms * 1500;
+    // the code) while all of them together are about a microsecond of the FP64 pipes, and
+    // for two or three products, which do not pay for turning a sum into a double
+    // (508870 x 2: 18.2 us in fixed point, 11.2 with a thread per output's Kahan sum)
+    p->fx = f64 && !p->mix && k.nq >= 4 && k.outputs * k.nq > (uint64_t)sms * 1500;
     const bool plain = f64 && !p->mix && !p->fx;
     const uint64_t lanes = (uint64_t)sms * 512;
     if (p->row) {
