@@ -112,6 +112,18 @@ template <typename T, bool KAHAN> struct Acc {
             s = fma(a, b, s);
         }
     }
+    // The same with the product's rounding error kept too (three instructions more): one of
+    // a block's products in this form makes up for what shorter sums lose at their start.
+    __device__ __forceinline__ void fma_add_exact(T a, T b)
+    {
+        if (KAHAN) {
+            const T y = fma(a, b, -c), r = fma(-a, b, y) + c, t = s + y;
+            c = ((t - s) - y) + r;
+            s = t;
+        } else {
+            s = fma(a, b, s);
+        }
+    }
     // Combine with another accumulator (order-fixed, compensated).
     __device__ __forceinline__ void merge(T os, T oc)
     {
