@@ -616,3 +616,24 @@ def test_thin_prefixes_stay_on_their_kernel_in_one_wave(engine):
                                (engine.BF16A, 8, 9, 200, gs), (engine.BF16A, 2, 32, 8000, gs),
                                (engine.F64, 2, 256, 200, thin), (engine.F64, 8, 200, 2, thin), (engine.F64, 8, 700, 2, gs)):
         assert _general(engine, dt, P, nq, S) == want, (dt, P, nq, S)
+
+
+def test_sizes_past_64_bits_are_told_in_full(engine):
+    """Layouts that span more than 64 bits' worth of bytes: the message gives the whole number."""
+    lists = [[4, 5, 6], [1, 4, 20], [1, 2, 3], [4], [5, 6], [2 ** 62, 2 ** 63], [1, 2]]
+    flat = [x for v in lists for x in v]
+    st = engine.library().tlibg_ttv_packed(_packed(engine, 0, 1, 3, (16, 32, 48), (480, 16, 120), flat))
+    assert st == engine.ERR_ARGUMENT
+    assert engine._last_error() == f"tlibg: buffer c holds 120 bytes, its layout addresses {4 * (1 + 4 * 2 ** 62 + 5 * 2 ** 63)}"
+
+
+def test_array_call_refuses_modes_as_before(engine):
+    """Modes that are no integers or out of range are refused before anything is allocated."""
+    import ctypes
+    import torch
+    A, b = torch.zeros(4, 5), torch.zeros(5)
+    with pytest.raises(ctypes.ArgumentError):
+        engine.ttv_array(1.0, A, b)
+    for q in (-1, 3, 9):
+        with pytest.raises((engine.TTVError, ValueError), match="mode"):
+            engine.ttv_array(q, A, b)

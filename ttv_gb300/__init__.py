@@ -492,16 +492,17 @@ def ttv_array(q, A, b, *, out=None, stream=None, **opts):
     na = list(A.shape)
     cdt = torch.float32 if A.dtype == torch.bfloat16 else A.dtype
     dt = BF16A if A.dtype == torch.bfloat16 else (F64 if A.dtype == torch.float64 else F32)
-    if p > 1 and q > 0 and 0 not in na:
-        c = torch.empty(na[:q - 1] + na[q:], dtype=cdt, device=A.device) if out is None else out
-        try:
+    words = None
+    try:
+        if p > 1 and q > 0 and 0 not in na:
+            c = torch.empty(na[:q - 1] + na[q:], dtype=cdt, device=A.device) if out is None else out
             words = _pack(dt, q, p, A, b, c, (A.nbytes, b.nbytes, c.nbytes), stream, opts, *na, *A.stride(),
                           b.shape[0])
-        except _UNPLAIN:
-            words = None
-        if words is not None:
-            _raise(library().tlibg_ttv_packed_rowmajor(words))
-            return c
+    except _UNPLAIN:
+        words = None
+    if words is not None:
+        _raise(library().tlibg_ttv_packed_rowmajor(words))
+        return c
     pia = list(range(p, 0, -1))
     wa = [s for s in A.stride()]
     nc = output_shape(na, q)

@@ -1147,30 +1147,39 @@ int check_elem_align(int dtype, const void* a, const void* b, const void* c)
     return TLIBG_OK;
 }
 
-// Elements a tensor with extents n and strides w spans (2^62 and more: 2^62).
-uint64_t addressed(const size_t* n, const size_t* w, size_t p)
+// Elements a tensor with extents n and strides w spans (past 128 bits: the largest).
+typedef unsigned __int128 wide_t;
+wide_t addressed(const size_t* n, const size_t* w, size_t p)
 {
-    constexpr uint64_t MOST = uint64_t(1) << 62;
-    uint64_t last = 0;
+    wide_t last = 0;
     for (size_t r = 0; r < p; ++r)
         if (n[r] == 0) return 0;
     for (size_t r = 0; r < p; ++r) {
-        uint64_t t;
-        if (mul_overflows(n[r] - 1, w[r], &t) || t >= MOST || (last += t) >= MOST) return MOST;
+        const wide_t t = (wide_t)(n[r] - 1) * w[r];
+        if (last > ~t - 1) return ~(wide_t)0;
+        last += t;
     }
     return last + 1;
 }
 
+std::string decimal(wide_t x)
+{
+    std::string s;
+    do s.insert(s.begin(), (char)('0' + (int)(x % 10)));
+    while (x /= 10);
+    return s;
+}
+
 // Buffers of known size (have[0..2]: a, b, c, in bytes or in elements) must hold what their layouts address; the kernels trust the
 // metadata as the reference does.
-int check_sizes(int dtype, const uint64_t* have, bool in_bytes, const uint64_t* need)
+int check_sizes(int dtype, const uint64_t* have, bool in_bytes, const wide_t* need)
 {
     const uint64_t es[3] = {elem_size_a(dtype), elem_size_t(dtype), elem_size_t(dtype)};
     for (int i = 0; i < 3; ++i) {
         if (have[i] == UINT64_MAX || (in_bytes ? have[i] / es[i] : have[i]) >= need[i]) continue;   // unknown, or enough
         std::string m = std::string("tlibg: buffer ") + "abc"[i] + " holds " + std::to_string(have[i]);
-        m += in_bytes ? " bytes, its layout addresses " + std::to_string(need[i] * es[i])
-                      : " elements, its strides address " + std::to_string(need[i]);
+        m += in_bytes ? " bytes, its layout addresses " + decimal(need[i] * es[i])
+                      : " elements, its strides address " + decimal(need[i]);
         return fail(TLIBG_ERR_ARGUMENT, m);
     }
     return TLIBG_OK;
@@ -1186,7 +1195,7 @@ int run_device(int dtype, size_t q, size_t p, const void* a, const size_t* na, c
     int st = analyse(q, p, a, na, wa, pia, b, nb, c, nc, wc, pic, &cn);
     if (st) return st;
     if (bytes) {
-        const uint64_t need[3] = {addressed(na, wa, p), nb[0], addressed(nc, wc, p - 1)};
+        const wide_t need[3] = {addressed(na, wa, p), nb[0], addressed(nc, wc, p - 1)};
         if ((st = check_sizes(dtype, bytes, true, need))) return st;
     }
     st = check_elem_align(dtype, a, b, c);
@@ -1470,7 +1479,7 @@ int tlibg_ttv_strided_packed(const uint64_t* w)
     const size_t* na = reinterpret_cast<const size_t*>(w + TLIBG_PACKED_WORDS);
     const size_t *wa = na + p, *pia = wa + p, *nb = pia + p, *nc = nb + 1, *wc = nc + (p - 1), *pic = wc + (p - 1),
                  *wb = pic + (p - 1);
-    const uint64_t need[3] = {addressed(na, wa, p), addressed(nb, wb, 1), p > 1 ? addressed(nc, wc, p - 1) : 0};
+    const wide_t need[3] = {addressed(na, wa, p), addressed(nb, wb, 1), p > 1 ? addressed(nc, wc, p - 1) : 0};
     if (int st = check_sizes(dtype, w + TLIBG_PACKED_BYTES, false, need)) return st;
     return tlibg_ttv_strided(dtype, q, p, ptr(TLIBG_PACKED_A), na, wa, pia, ptr(TLIBG_PACKED_B), nb, wb[0],
                              ptr(TLIBG_PACKED_C), nc, wc, pic, ptr(TLIBG_PACKED_STREAM));
