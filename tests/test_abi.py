@@ -637,3 +637,15 @@ def test_array_call_refuses_modes_as_before(engine):
     for q in (-1, 3, 9):
         with pytest.raises((engine.TTVError, ValueError), match="mode"):
             engine.ttv_array(q, A, b)
+
+
+def test_small_buffers_are_told_before_unsupported_strides(engine):
+    """A call that is both too small and not dense is refused for its buffer, as the general form does."""
+    na, wa, c = [4, 5, 6], [1, 8, 40], [5, 6]
+    flat = [x for v in (na, wa, [1, 2, 3], [4], c, [1, 5], [1, 2]) for x in v]
+    need = 4 * (1 + 3 + 4 * 8 + 5 * 40)
+    call = engine.library().tlibg_ttv_packed
+    assert call(_packed(engine, 0, 1, 3, (16, 32, 48), (480, 16, 120), flat)) == engine.ERR_ARGUMENT
+    assert engine._last_error() == f"tlibg: buffer a holds 480 bytes, its layout addresses {need}"
+    assert call(_packed(engine, 0, 1, 3, (16, 32, 48), (need, 16, 120), flat)) == engine.ERR_UNSUPPORTED
+    assert "dense tensor A" in engine._last_error()

@@ -1193,11 +1193,11 @@ int run_device(int dtype, size_t q, size_t p, const void* a, const size_t* na, c
     NvtxRange nvtx("tlibg_ttv");
     Canon cn;
     int st = analyse(q, p, a, na, wa, pia, b, nb, c, nc, wc, pic, &cn);
-    if (st) return st;
-    if (bytes) {
+    if (bytes && (st == TLIBG_OK || st == TLIBG_ERR_UNSUPPORTED)) {   // sizes before what only this engine refuses
         const wide_t need[3] = {addressed(na, wa, p), nb[0], addressed(nc, wc, p - 1)};
-        if ((st = check_sizes(dtype, bytes, true, need))) return st;
+        if (int small = check_sizes(dtype, bytes, true, need)) return small;
     }
+    if (st) return st;
     st = check_elem_align(dtype, a, b, c);
     if (st) return st;
     DevInfo d = dev_info();
