@@ -153,7 +153,9 @@ struct BShape {
 };
 
 // The unit's lanes per row or warps along q: the variant's, and more while the
-// unit's chain of loads is longer than the shape allows.  A trip is 4 rows of a
+// unit's chain of loads is longer than the shape allows; `nq` is the whole
+// contraction also for variants that cut it into segments, which so get more
+// warps than their shorter chains need.  A trip is 4 rows of a
 // 16-byte column, 12 or 8 of a narrow one, 16 elements of a row's lane.
 __host__ __device__ inline uint64_t unit_trips(int kind, int group, int vec, uint64_t rows)
 {

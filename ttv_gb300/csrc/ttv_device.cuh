@@ -145,8 +145,8 @@ template <typename T, bool KAHAN> struct Acc {
 // One Kahan step of two fp32 sums in packed instructions (two lanes each, the
 // results of the scalar step bit for bit): with m = c - a b = -(a b - c),
 // t = s - m and c = (t - s) + m.  Two instructions an element instead of four,
-// which is what bf16 storage was short of (device time: 16 x 2^20 x 16 95.5 ->
-// 92.7 us, rows of 64 40.7 -> 36.7, of 645 34.6 -> 32.9; fp32 level to 3 %).
+// which is what bf16 storage was short of (device time: rows of 64 40.7 -> 36.7 us,
+// of 645 34.6 -> 32.9; 16 x 2^20 x 16 95.5, level; fp32 level to 3 %).
 __device__ __forceinline__ void kahan_pair(Acc<float, true>& p, Acc<float, true>& q, float a0, float a1, float b0, float b1)
 {
     asm("{\n\t"

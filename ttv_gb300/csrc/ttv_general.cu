@@ -47,8 +47,9 @@ namespace tlibg {
 // lives off warps in flight: 6 for one-element columns (38 x 814,000 outputs:
 // 30.9 us, 42 when the shared form's code held it to 4), 4 for 16-byte columns
 // (5 spills into the loop: 25.2 -> 30.0 us on 33 x 889,000; 3 for bf16 ones: 256 x
-// 1024 x 512 50.6 -> 57.8).  The fp64 kernels
-// hold 128-bit sums: 4 and 3, with the spills outside the loops (2 and 2 were
+// 1024 x 512 50.6 -> 57.8).  Shared 16-byte and two-vector kernels spill 4 to 64
+// bytes, bf16 ones with an exact start up to 160.  The fp64 kernels
+// hold 128-bit sums: 4 and 3, with the spills (24 to 344 bytes) outside the loops (2 and 2 were
 // 3 to 30 % slower).
 template <typename T, int N, bool SHARE> constexpr int gs_col_ctas()
 {
@@ -949,7 +950,8 @@ void gs_plan(int sms, GSPlan* p, bool segments)
         k.group_log2 = gl;
         const uint64_t lane_rows = (nv + (1u << gl) - 1) >> gl;
         // rows per group: several where a row is only a load or two per lane
-        // (16-byte fp32 vectors: two at most, four spill; bf16 ones hold eight sums already)
+        // (16-byte fp32 vectors: two at most, which spill 24 bytes, 60 with an exact start; bf16
+        // ones hold eight sums already)
         p->M = plain || p->mix || lane_rows > 4 || p->V == 8 ? 1 : (lane_rows > 2 || p->V == 4 ? 2 : 4);
         while (p->M > 1 && (k.outputs << gl) < lanes * p->M) p->M /= 2;
         gs_split(p, lane_rows, gl == 5, segments, (uint32_t)((32u >> gl) * p->M), p->V * p->M, sms);

@@ -12,7 +12,7 @@
 //
 // Loss: L = (1/n) sum_s 0.5 (f(x_s) - y_s)^2 over the minibatch.
 //
-// What bounds them: nothing the chip has; a minibatch of 512 is 59 MFLOP and
+// What bounds them: nothing the chip has; a minibatch of 512 is 29 MFLOP and
 // 35 KB of input beside 38 KB of parameters.  It is latency, so the work is
 // spread until every chain is short: one thread per sample (17,000 dependent
 // FMAs, weights read from L1 one word at a time) took 430 us for 512 rows and
